@@ -9,6 +9,7 @@ import ctypes
 import glob
 import os
 import shutil
+import struct
 import subprocess
 from typing import Optional, Sequence
 
@@ -49,6 +50,16 @@ class _Dims(ctypes.Structure):
                 ("dk", ctypes.c_int32), ("dv", ctypes.c_int32), ("block_size", ctypes.c_int32),
                 ("flags", ctypes.c_int32), ("head_decays", ctypes.POINTER(ctypes.c_double)),
                 ("workspace", ctypes.c_void_p), ("workspace_bytes", ctypes.c_int64)]
+
+
+class _TokenDims(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_int32) for n in ("layers", "B", "H", "dk", "dv", "ffn", "prev_dtype", "out_dtype")] + \
+               [("head_decays", ctypes.POINTER(ctypes.c_double)), ("workspace", ctypes.c_void_p), ("workspace_bytes", ctypes.c_int64)]
+
+
+# fpb_decoder_layer: 19 pointers, s_prev and its strides, s_out and its strides, two activation codes, three epsilons
+DECODER_LAYER = struct.Struct("19Q Q2q Q2q 2q 3d")
+ACT_SWISH, ACT_GELU, ACT_RELU = 1, 2, 3
 
 
 def sources() -> list[str]:
@@ -109,6 +120,8 @@ _SIGNATURES = {
                            ctypes.c_void_p, _SEQ_P, _SEQ_P, _SEQ_P, _SEQ_P, _STATE_P, ctypes.c_void_p,
                            ctypes.c_void_p],
     "fpb_retention_step": [_DIMS_P, ctypes.c_int32, _SEQ_P, _SEQ_P, _SEQ_P, _STATE_P, _SEQ_P, _STATE_P, ctypes.c_void_p],
+    "fpb_decoder_token": [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int64,
+                          ctypes.c_void_p],
     "fpb_rotary": [ctypes.c_int32] * 7 + [ctypes.c_void_p, ctypes.c_int64, _SEQ_P, _SEQ_P, _SEQ_P, _SEQ_P, ctypes.c_void_p],
     "fpb_groupnorm_gate_fwd": [ctypes.c_int32] * 5 + [ctypes.c_float, ctypes.c_int32, _SEQ_P, _SEQ_P, _SEQ_P, ctypes.c_void_p],
     "fpb_groupnorm_gate_bwd": [ctypes.c_int32] * 5 + [ctypes.c_float, ctypes.c_int32, _SEQ_P, _SEQ_P, _SEQ_P, _SEQ_P, _SEQ_P,
@@ -155,7 +168,7 @@ _DIAG_SIGNATURES = {
 def exported_symbols() -> list[str]:
     """Every entry point include/flash_pop_b200.h declares."""
     return list(_SIGNATURES) + ["fpb_strerror", "fpb_version", "fpb_last_path", "fpb_last_cuda_error",
-                                "fpb_launch_count", "fpb_workspace_bytes"]
+                                "fpb_launch_count", "fpb_workspace_bytes", "fpb_decoder_token_workspace"]
 
 
 def _load(path: str) -> ctypes.CDLL:
@@ -176,6 +189,8 @@ def _load(path: str) -> ctypes.CDLL:
     handle.fpb_launch_count.restype = ctypes.c_int64
     handle.fpb_workspace_bytes.argtypes = [_DIMS_P]
     handle.fpb_workspace_bytes.restype = ctypes.c_int64
+    handle.fpb_decoder_token_workspace.argtypes = [ctypes.POINTER(_TokenDims)]
+    handle.fpb_decoder_token_workspace.restype = ctypes.c_int64
     return handle
 
 

@@ -399,6 +399,35 @@ int fpb_retention_step(const fpb_dims* dims, int32_t state_dtype, const fpb_seq*
   return finish_launches(1, FPB_PATH_SIMT);
 }
 
+int64_t fpb_decoder_token_workspace(const fpb_token_dims* dims) {
+  if (!dims) return 0;
+  fpb_token_dims d = *dims;
+  d.layers = 0;                                    // shape limits only
+  return check_decoder_token(d, nullptr) == FPB_OK && d.B > 0 ? decoder_token_workspace(d) : 0;
+}
+
+int fpb_decoder_token(const fpb_token_dims* dims, const fpb_decoder_layer* layers, const void* x, int64_t x_stride, void* y,
+                      int64_t y_stride, fpb_stream_t stream) {
+  if (!dims) return FPB_ERR_NULL_POINTER;
+  FPB_TRY(check_decoder_token(*dims, layers));
+  if (dims->layers == 0 || dims->B == 0) return FPB_OK;
+  const int64_t width = (int64_t)dims->H * dims->dv;
+  if (!x || !y) return FPB_ERR_NULL_POINTER;
+  if ((uintptr_t)x % 16 || x_stride % 8 || (uintptr_t)y % 4 || y_stride % 2) return FPB_ERR_BAD_STRIDE;
+  if (dims->B > 1 && (x_stride < width || y_stride < width)) return FPB_ERR_BAD_STRIDE;
+  float gamma[FPB_MAX_HEADS];
+  for (int h = 0; h < dims->H; ++h) {
+    const double g = dims->head_decays[h];
+    if (!std::isfinite(g) || g < 0.0 || g > 1.0) return FPB_ERR_BAD_DECAY;
+    gamma[h] = (float)g;
+  }
+  FPB_TRY(check_device());
+  int n_launched = 0;
+  const int r = launch_decoder_token(*dims, layers, gamma, x, x_stride, y, y_stride, (cudaStream_t)stream, &n_launched);
+  const int f = finish_launches(n_launched, FPB_PATH_SIMT);
+  return r != FPB_OK ? r : f;
+}
+
 namespace {
 // shapes and alignment of a (B,T,H,d) tensor read or written `vec` elements at a time
 int check_plain_seq(const fpb_seq* s, int dtype, int B, int T, int H, int d, int vec_bytes) {

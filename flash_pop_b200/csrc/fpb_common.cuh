@@ -54,6 +54,12 @@ int launch_walk(const WalkParams& p, int dtype, bool state_f32, int B, cudaStrea
 int launch_retention_step(int dtype, int state_dtype, int B, int H, int dk, int dv, const float* gamma, SeqView q,
                           SeqView k, SeqView v, SeqView o, StateView s_prev, StateView s_out, cudaStream_t stream);
 
+// One token through a stack of decoder layers (decode_token.cu).
+int64_t decoder_token_workspace(const fpb_token_dims& d);
+int check_decoder_token(const fpb_token_dims& d, const fpb_decoder_layer* layers);
+int launch_decoder_token(const fpb_token_dims& d, const fpb_decoder_layer* layers, const float* gamma, const void* x, int64_t x_stride,
+                         void* y, int64_t y_stride, cudaStream_t stream, int* n_launched);
+
 // Fused elementwise passes around the operator (layer_fused.cu).
 int launch_rotary(int in_dtype, int out_dtype, int B, int T, int H, int d, bool conjugate, const float* phasors,
                   int64_t phasor_stride_b, const SeqView in[2], const SeqView out[2], int n_tensors, cudaStream_t stream);

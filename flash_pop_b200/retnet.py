@@ -28,6 +28,7 @@ from torch import Tensor
 from flash_pop_b200.fused_retention import cuda_core_kernels, fused_chunk_retention, retention_step
 from flash_pop_b200.layer_ops import groupnorm_gate, groupnorm_gate_supported, norm_in_fp32
 from flash_pop_b200.recurrent_state import RecurrentState
+from flash_pop_b200.token_stack import decoder_token
 from flash_pop_b200.xpos_emb import XPos
 
 ActivationString = Literal["swish", "gelu", "relu"]
@@ -308,6 +309,9 @@ class RetNetDecoder(nn.Module):
         return x, RecurrentState(torch.stack(states), rs.index + advance)
 
     def forward_recurrent(self, x: Tensor, recurrent_state: RecurrentState = None) -> Tuple[Tensor, RecurrentState]:
+        fused = decoder_token(self, x, recurrent_state, RetNetDecoderLayer, MultiScaleRetention)
+        if fused is not None:
+            return fused
         return self._walk_layers(x, recurrent_state, lambda layer, h, idx, st: layer.forward_recurrent(h, idx, st), 1)
 
     def forward_chunkwise(self, x: Tensor, recurrent_state: RecurrentState = None) -> Tuple[Tensor, RecurrentState]:

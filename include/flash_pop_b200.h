@@ -199,6 +199,42 @@ int fpb_retention_step(const fpb_dims* dims, int32_t state_dtype, const fpb_seq*
                        const fpb_seq* v, const fpb_state* s_prev, const fpb_seq* o, const fpb_state* s_out,
                        fpb_stream_t stream);
 
+/* Activations of a decoder layer (flash_pop/retnet.py:21-38): x sigmoid(x), x Phi(x), max(x, 0), or none. */
+enum { FPB_ACT_NONE = 0, FPB_ACT_SWISH = 1, FPB_ACT_GELU = 2, FPB_ACT_RELU = 3 };
+
+/* One pre-norm decoder layer as fpb_decoder_token reads it.  Matrices are bf16, row-major (out, in), 16-byte aligned;
+ * biases bf16 (NULL: none); norm parameters fp32 (NULL: 1 and 0). */
+typedef struct fpb_decoder_layer {
+  const float *norm1_w, *norm1_b, *norm2_w, *norm2_b;
+  const void *wq, *bq, *wk, *bk, *wv, *bv, *wg, *bg;   /* (H dk, H dv), (H dk, H dv), (H dv, H dv), (H dv, H dv) */
+  const void *wo, *bo, *w1, *b1, *w2, *b2;             /* (H dv, H dv), (ffn, H dv), (H dv, ffn) */
+  const float* phasors;                                /* dk / 2 pairs (cos, sin) of the token's position; NULL: no rotation */
+  const void* s_prev; int64_t prev_sb, prev_sh;        /* (B, H, dk, dv) of prev_dtype, NULL: zeros */
+  void* s_out; int64_t out_sb, out_sh;                 /* (B, H, dk, dv) of out_dtype; may not overlap any s_prev */
+  int64_t act_gate, act_ffn;                           /* FPB_ACT_* of the retention's gate and of the feed-forward */
+  double norm1_eps, norm2_eps, gn_eps;
+} fpb_decoder_layer;
+
+typedef struct fpb_token_dims {
+  int32_t layers, B, H, dk, dv, ffn;
+  int32_t prev_dtype, out_dtype;                       /* element types of the states */
+  const double* head_decays;                           /* host, H entries, shared by the layers */
+  void* workspace; int64_t workspace_bytes;            /* device, 16-byte aligned, fpb_decoder_token_workspace bytes */
+} fpb_token_dims;
+
+/* Scratch bytes of fpb_decoder_token for these dims; 0 when they are out of its range. */
+int64_t fpb_decoder_token_workspace(const fpb_token_dims* dims);
+
+/*
+ * One token of every row through `layers` consecutive decoder layers (RetNetDecoder.forward_recurrent,
+ * flash_pop/retnet.py:535-546; RetNetDecoderLayer.forward_recurrent and MultiScaleRetention.forward_recurrent below it):
+ *   x <- x + out_proj(GroupNorm(retention step(rotate(q), rotate(k), v)) . act(gate)),   x <- x + linear2(act(linear1(norm(x))))
+ * x, y: (B, H dv) bf16 rows, row pitches in elements.  At most 64 rows, H dv <= 1024 and a multiple of 32, ffn a multiple
+ * of 32, H dk of 8, dv of 4, dk even; FPB_ERR_BAD_SHAPE outside.  Five launches per layer, no allocation, no synchronisation.
+ */
+int fpb_decoder_token(const fpb_token_dims* dims, const fpb_decoder_layer* layers, const void* x, int64_t x_stride,
+                      void* y, int64_t y_stride, fpb_stream_t stream);
+
 /*
  * The two elementwise passes of a retention layer either side of the operator, each as one streaming kernel
  * (fp32 arithmetic).  They replace PyTorch expressions of the reference rather than kernels of its own.
