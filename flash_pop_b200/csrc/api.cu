@@ -148,6 +148,14 @@ void fill_common(WalkParams& p, const Call& c, int dir, const SuffixStates& sfx)
 void own_is_dv(WalkParams& p, const Call& c) { p.n_own = c.dv; p.n_red = c.dk; p.x_stride_red = c.dv; p.x_stride_own = 1; }
 void own_is_dk(WalkParams& p, const Call& c) { p.n_own = c.dk; p.n_red = c.dv; p.x_stride_red = 1; p.x_stride_own = c.dv; }
 
+ChunkArgs chunk_args(const Call& c, int64_t batch, SeqView q, SeqView k, SeqView v, StateView s0) {
+  ChunkArgs a{};
+  a.q = q; a.k = k; a.v = v; a.s0 = s0; a.gamma = c.gamma;
+  a.B = (int)batch; a.T = c.T; a.H = c.H; a.dk = c.dk; a.dv = c.dv;
+  a.scratch = c.scratch; a.scratch_bytes = c.scratch_bytes;
+  return a;
+}
+
 // ---- forward (plain, POP, suffix) --------------------------------------------------------------
 int forward(const Call& c, int64_t batch, SeqView q, SeqView k, SeqView v, StateView s0, SeqView o, StateView s_out,
             void* block_states, SuffixStates sfx, cudaStream_t stream) {
@@ -163,6 +171,14 @@ int forward(const Call& c, int64_t batch, SeqView q, SeqView k, SeqView v, State
     const int r = launch_umma_fwd(a, stream, &n_launched);
     if (r == FPB_OK) return finish_launches(n_launched, FPB_PATH_TCGEN05);
     if (r != FPB_UMMA_NOT_APPLICABLE) return r;
+  }
+  if (c.dtype == FPB_F32 && !block_states && sfx.M == 0) {
+    ChunkArgs a = chunk_args(c, batch, q, k, v, s0);
+    a.o = o; a.s_out = s_out;
+    int n_launched = 0;
+    const int r = launch_chunk_fwd(a, stream, &n_launched);
+    if (r == FPB_OK) return finish_launches(n_launched, FPB_PATH_SIMT);
+    if (r != FPB_CHUNK_NOT_APPLICABLE) { tl_last_cuda_error = (int)cudaGetLastError(); return r; }
   }
   WalkParams p;
   fill_common(p, c, +1, sfx);
@@ -192,6 +208,14 @@ int backward(const Call& c, int64_t batch, SeqView q, SeqView k, SeqView v, Stat
     const int r = launch_umma_bwd(a, stream, &n_launched);
     if (r == FPB_OK) return finish_launches(n_launched, FPB_PATH_TCGEN05);
     if (r != FPB_UMMA_NOT_APPLICABLE) return r;
+  }
+  if (c.dtype == FPB_F32 && c.block_size == 0 && sfx_in.M == 0) {
+    ChunkArgs a = chunk_args(c, batch, q, k, v, s0);
+    a.dO = dO; a.dQ = dQ; a.dK = dK; a.dV = dV; a.d_s_out = d_s_out; a.d_s0 = d_s0;
+    int n_launched = 0;
+    const int r = launch_chunk_bwd(a, (c.flags & FPB_FLAG_SKIP_DQ) != 0, (c.flags & FPB_FLAG_SKIP_DKDV) != 0, stream, &n_launched);
+    if (r == FPB_OK) return finish_launches(n_launched, FPB_PATH_SIMT);
+    if (r != FPB_CHUNK_NOT_APPLICABLE) { tl_last_cuda_error = (int)cudaGetLastError(); return r; }
   }
   WalkParams p;
   int r, n = 0;
@@ -253,8 +277,9 @@ int fpb_retention_fwd_static(const fpb_dims* dims, const fpb_seq* q, const fpb_s
   FPB_TRY(check_seq(c, v, c.dv, c.B)); FPB_TRY(check_seq(c, o, c.dv, c.B));
   FPB_TRY(check_state(s0, c)); FPB_TRY(check_state(s_out, c));
   FPB_TRY(check_device());
-  // a shape whose full split needs more than the built-in scratch holds is refused rather than split less
-  if (fpb_workspace_bytes(dims) > (int64_t)FPB_STATIC_SCRATCH_BYTES) return FPB_ERR_TOO_LARGE;
+  // a shape whose full split needs more than the built-in scratch holds is refused rather than split less (fp32 calls,
+  // whose kernels take any amount, split as far as it goes)
+  if (dims->dtype == FPB_BF16 && fpb_workspace_bytes(dims) > (int64_t)FPB_STATIC_SCRATCH_BYTES) return FPB_ERR_TOO_LARGE;
   float* scratch = static_scratch_ptr();
   if (!scratch) { tl_last_cuda_error = (int)cudaErrorInvalidSymbol; return FPB_ERR_LAUNCH; }
   c.scratch = scratch;
@@ -672,7 +697,9 @@ int fpb_version(void) { return 200; }
 int64_t fpb_workspace_bytes(const fpb_dims* dims) {
   // what lets the emptiest pass of this shape (one CTA per batch row and head) split as far as it would
   if (!dims || dims->B <= 0 || dims->H <= 0 || dims->T <= 0 || dims->dk <= 0 || dims->dv <= 0) return 0;
-  if (dims->dtype != FPB_BF16 || check_device() != FPB_OK) return 0;
+  if (check_device() != FPB_OK) return 0;
+  if (dims->dtype == FPB_F32) return dims->block_size > 0 ? 0 : chunk_f32_workspace(dims->B, dims->T, dims->H, dims->dk, dims->dv);
+  if (dims->dtype != FPB_BF16) return 0;
   // (the small state tiles run two CTAs per SM: ask for what that residency can use)
   const int ctas_per_sm = (dims->dk <= 64 || dims->dv <= 64) ? 2 : 1;
   const Segments sg = choose_segments((long long)dims->B * dims->H, ctas_per_sm, dims->T, 64, (long long)dims->B * dims->H,

@@ -50,6 +50,21 @@ struct WalkParams {
 // `state_f32`: the states (x0, x_out, block states, suffix start states) are fp32 whatever the activations are
 int launch_walk(const WalkParams& p, int dtype, bool state_f32, int B, cudaStream_t stream);
 
+// Chunked fp32 kernels (chunk_f32.cu): plain forward and backward of fp32 calls.  FPB_CHUNK_NOT_APPLICABLE sends the call
+// to the token walk (head dimensions above 128 or not a multiple of 4, tensors that 16-byte accesses cannot read, very
+// short sequences).  `scratch` (may be null) holds the T-segments' states, chunk_f32_workspace bytes for the full split.
+constexpr int FPB_CHUNK_NOT_APPLICABLE = -1;
+struct ChunkArgs {
+  SeqView q, k, v, dO, o, dQ, dK, dV;
+  StateView s0, s_out, d_s_out, d_s0;
+  const float* gamma;                                   // host, H entries
+  int B, T, H, dk, dv;
+  float* scratch; int64_t scratch_bytes;
+};
+int64_t chunk_f32_workspace(int B, int T, int H, int dk, int dv);
+int launch_chunk_fwd(const ChunkArgs& a, cudaStream_t stream, int* n_launched);
+int launch_chunk_bwd(const ChunkArgs& a, bool skip_dq, bool skip_dkdv, cudaStream_t stream, int* n_launched);
+
 // One recurrent decoding step (retention_step.cu); `dtype` is that of q, k, v, o, `state_dtype` that of the states.
 int launch_retention_step(int dtype, int state_dtype, int B, int H, int dk, int dv, const float* gamma, SeqView q,
                           SeqView k, SeqView v, SeqView o, StateView s_prev, StateView s_out, cudaStream_t stream);
