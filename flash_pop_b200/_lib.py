@@ -7,10 +7,14 @@ from __future__ import annotations
 
 import ctypes
 import glob
+import importlib.machinery
+import importlib.util
 import os
 import shutil
 import struct
 import subprocess
+import sys
+import sysconfig
 from typing import Optional, Sequence
 
 import torch
@@ -22,6 +26,9 @@ LIB_PATH = os.path.join(LIB_DIR, "libflash_pop_b200.so")
 # the same sources with -DFPB_DIAGNOSTICS: adds the fpb_debug_* hooks (schedule choices, wait limit, time stamps) that
 # some tests use; the operators never load it on their own
 DIAG_LIB_PATH = os.path.join(LIB_DIR, "libflash_pop_b200_diag.so")
+
+# argument checks, allocations and calls of the operators' host side
+NATIVE_SOURCE = os.path.join(PKG_DIR, "native", "fast_calls.cpp")
 
 NVCC_FLAGS = [
     "-std=c++17", "-O3", "-lineinfo",
@@ -75,9 +82,31 @@ def _stale(path: str = LIB_PATH) -> bool:
     return any(os.path.getmtime(p) > built for p in deps)
 
 
+def _native_path() -> str:
+    """The host-side extension (native/fast_calls.cpp); it depends on the torch and Python it was compiled against."""
+    return os.path.join(LIB_DIR, f"fpb_fast_calls-{torch.__version__}-{sys.implementation.cache_tag}.so")
+
+
+def _native_command(out: str) -> list[str]:
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"))), "include")
+    include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+               sysconfig.get_paths()["include"], cuda]
+    lib = os.path.join(root, "lib")
+    return [shutil.which("g++") or "g++", "-std=c++17", "-O2", "-fPIC", "-shared", *(f"-I{d}" for d in include),
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", NATIVE_SOURCE, "-o", out, f"-L{lib}", f"-Wl,-rpath,{lib}",
+            "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+
+
+def _native_stale() -> bool:
+    path = _native_path()
+    deps = [NATIVE_SOURCE, *glob.glob(os.path.join(PKG_DIR, "..", "include", "*.h"))]
+    return not os.path.exists(path) or any(os.path.getmtime(p) > os.path.getmtime(path) for p in deps)
+
+
 def build(force: bool = False, verbose: bool = False, diagnostics: bool = True) -> str:
-    """Compile every CUDA source of the package for sm_100a into one shared library, in-tree; with `diagnostics`
-    also the diagnostics build of the same sources.  Returns the path of the release library."""
+    """Compile every CUDA source of the package for sm_100a into one shared library, in-tree, and the host-side extension
+    beside it; with `diagnostics` also the diagnostics build of the CUDA sources.  Returns the path of the release library."""
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     os.makedirs(LIB_DIR, exist_ok=True)
     jobs = [(LIB_PATH, [])] + ([(DIAG_LIB_PATH, ["-DFPB_DIAGNOSTICS"])] if diagnostics else [])
@@ -91,12 +120,15 @@ def build(force: bool = False, verbose: bool = False, diagnostics: bool = True) 
             cmd.insert(1, "-Xptxas=-v")
             print(" ".join(cmd))
         procs.append((path, tmp, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.PIPE, text=True)))
+    if force or _native_stale():
+        tmp = _native_path() + ".partial"
+        procs.append((_native_path(), tmp, subprocess.Popen(_native_command(tmp), stdout=subprocess.PIPE, stderr=subprocess.PIPE, text=True)))
     for path, tmp, proc in procs:
         out, err = proc.communicate()
         if proc.returncode != 0:
             if os.path.exists(tmp):
                 os.remove(tmp)
-            raise RuntimeError("nvcc failed:\n" + out + err)
+            raise RuntimeError("compiler failed:\n" + out + err)
         os.replace(tmp, path)
         if verbose:
             print(err)
@@ -199,6 +231,41 @@ def lib() -> ctypes.CDLL:
     if _lib is None:
         _lib = _load(LIB_PATH)
     return _lib
+
+
+# entry points of the C ABI that the host-side extension calls, in the order of its table
+_NATIVE_ENTRIES = ("fpb_retention_fwd", "fpb_retention_bwd", "fpb_pop_retention_fwd", "fpb_pop_retention_bwd", "fpb_pop_suffix_fwd",
+                   "fpb_pop_suffix_bwd", "fpb_retention_step", "fpb_workspace_bytes", "fpb_rotary", "fpb_groupnorm_gate_fwd",
+                   "fpb_groupnorm_gate_bwd", "fpb_layernorm_fwd", "fpb_layernorm_bwd")
+_native = None
+_native_bound: Optional[ctypes.CDLL] = None
+
+
+def native():
+    """The host-side extension, calling into the library that lib() gives.  Its functions return None for calls they leave
+    to the Python path, a nonzero int for a status of the C ABI (see `check`), else their results."""
+    global _native, _native_bound
+    if _native is None:
+        path = _native_path()
+        if not os.path.exists(path):
+            raise RuntimeError(f"{path} is missing: build it with `python -c 'import flash_pop_b200; flash_pop_b200.build()'`")
+        loader = importlib.machinery.ExtensionFileLoader("fpb_fast_calls", path)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("fpb_fast_calls", path, loader=loader))
+        loader.exec_module(module)
+        _native = module
+    if _native_bound is not _lib or _lib is None:
+        handle = lib()
+        _native.bind(*(ctypes.cast(getattr(handle, n), ctypes.c_void_p).value for n in _NATIVE_ENTRIES))
+        _native_bound = handle
+    return _native
+
+
+def result(fast):
+    """The results of a native call, or None where it left the call to the Python path; raises on a status."""
+    if fast is None or type(fast) is tuple:
+        return fast
+    check(fast)
+    raise RuntimeError(f"flash_pop_b200: unexpected status {fast}")
 
 
 _diag: Optional[ctypes.CDLL] = None

@@ -69,6 +69,15 @@ class FusedChunkRetention(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, s, head_decays: Sequence[float], state_dtype: Optional[torch.dtype] = None):
+        if q.is_cuda:
+            fast = _lib.result(_lib.native().forward(q, k, v, s, head_decays, state_dtype, _flags(), 0))
+            if fast is not None:
+                sdt = fast[1].dtype
+                ctx.save_for_backward(q, k, v, s)
+                ctx.head_decays, ctx.state_dtype = head_decays, sdt
+                ctx.flags = _flags() | (_lib.FLAG_STATE_F32 if sdt != q.dtype else 0)
+                ctx.set_materialize_grads(False)
+                return fast
         head_decays = tuple(float(g) for g in head_decays)
         q, k, v, s = _prepare(q, k, v, s, head_decays)
         B, T, H, dk = q.shape
@@ -93,6 +102,12 @@ class FusedChunkRetention(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dO, dS_new):
         q, k, v, s = ctx.saved_tensors
+        need = ctx.needs_input_grad
+        need_s = s is not None and need[3]
+        fast = _lib.result(_lib.native().backward(q, k, v, s, dO, dS_new, ctx.head_decays, ctx.state_dtype, ctx.flags, 0,
+                                                  need[0], need[1] or need[2] or need_s, need_s))
+        if fast is not None:
+            return *fast, None, None
         B, T, H, dk = q.shape
         dv = v.shape[-1]
         if dO is None:
@@ -150,6 +165,11 @@ def retention_step(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, head_decay
     q, k: (B, H, dk); v: (B, H, dv); prev_state: (B, H, dk, dv) or None (zeros).  Returns (o (B, H, dv), state).
     The state's element type is ``state_dtype``, else that of ``prev_state``, else that of q; with ``in_place`` the
     new state overwrites ``prev_state``.  Inference only: no gradient is recorded."""
+    if q.is_cuda:
+        decays = head_decays if type(head_decays) is tuple else tuple(float(g) for g in head_decays)
+        fast = _lib.result(_lib.native().step(q, k, v, decays, prev_state, state_dtype, bool(in_place)))
+        if fast is not None:
+            return fast
     _lib.require_cuda(q, k, v, prev_state)
     if q.dim() != 3 or k.shape != q.shape or v.dim() != 3 or v.shape[:2] != q.shape[:2]:
         raise ValueError(f"expected q,k (B,H,dk) and v (B,H,dv); got {tuple(q.shape)}, {tuple(k.shape)}, {tuple(v.shape)}")

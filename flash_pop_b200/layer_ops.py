@@ -27,6 +27,9 @@ def rotary_supported(q: Tensor) -> bool:
 
 
 def _rotate(q: Tensor, k: Optional[Tensor], phasors: Tensor, conjugate: bool, out_dtype: torch.dtype):
+    fast = _lib.result(_lib.native().rotary(q, k, phasors, conjugate, out_dtype))
+    if fast is not None:
+        return fast
     B, T, H, d = q.shape
     rows = phasors.shape[0]
     assert phasors.dtype == torch.float32 and phasors.is_contiguous() and tuple(phasors.shape[1:]) == (T, d // 2, 2)
@@ -75,6 +78,11 @@ def groupnorm_gate_supported(o: Tensor, z: Tensor) -> bool:
 class GroupNormGate(torch.autograd.Function):
     @staticmethod
     def forward(ctx, o, z, eps: float, swish: bool):
+        ctx.eps, ctx.swish = float(eps), bool(swish)
+        fast = _lib.result(_lib.native().gate_forward(o, z, ctx.eps, ctx.swish))
+        if fast is not None:
+            ctx.save_for_backward(o, z)
+            return fast[0]
         nb = 4 if o.dtype == torch.bfloat16 else 8
         o, z = _aligned(o, nb), _aligned(z, nb)
         B, T, H, dv = o.shape
@@ -83,12 +91,14 @@ class GroupNormGate(torch.autograd.Function):
             _lib.check(_lib.lib().fpb_groupnorm_gate_fwd(B, T, H, dv, _lib.dtype_code(o), float(eps), int(swish),
                                                          _lib.seq(o), _lib.seq(z), _lib.seq(y), _lib.stream_ptr(o.device)))
         ctx.save_for_backward(o, z)
-        ctx.eps, ctx.swish = float(eps), bool(swish)
         return y
 
     @staticmethod
     def backward(ctx, dy):
         o, z = ctx.saved_tensors
+        fast = _lib.result(_lib.native().gate_backward(o, z, dy, ctx.eps, ctx.swish))
+        if fast is not None:
+            return *fast, None, None
         B, T, H, dv = o.shape
         dy = _aligned(dy.to(o.dtype), 4 if o.dtype == torch.bfloat16 else 8)
         d_o, d_z = torch.empty_like(o, memory_format=torch.contiguous_format), torch.empty_like(z, memory_format=torch.contiguous_format)
@@ -128,6 +138,13 @@ def _ptr(t: Optional[Tensor]):
 class FusedLayerNorm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, eps: float):
+        ctx.eps, ctx.shape = float(eps), x.shape
+        ctx.w_dtype = None if weight is None else weight.dtype
+        ctx.b_dtype = None if bias is None else bias.dtype
+        fast = _lib.result(_lib.native().norm_forward(x, weight, bias, ctx.eps))
+        if fast is not None:
+            ctx.save_for_backward(x, weight)
+            return fast[0]
         x2 = _rows(x)
         rows, d = x2.shape
         w = None if weight is None else weight.detach().float().contiguous()
@@ -137,19 +154,21 @@ class FusedLayerNorm(torch.autograd.Function):
             _lib.check(_lib.lib().fpb_layernorm_fwd(rows, d, _lib.dtype_code(x2), float(eps), _ptr(x2), x2.stride(0) if rows > 1 else d,
                                                     _ptr(w), _ptr(b), _ptr(y), d, _lib.stream_ptr(x.device)))
         ctx.save_for_backward(x2, w)
-        ctx.eps, ctx.shape = float(eps), x.shape
-        ctx.w_dtype = None if weight is None else weight.dtype
-        ctx.b_dtype = None if bias is None else bias.dtype
         return y.view(x.shape)
 
     @staticmethod
     def backward(ctx, dy):
         x2, w = ctx.saved_tensors
+        need_w = ctx.w_dtype is not None and ctx.needs_input_grad[1]
+        need_b = ctx.b_dtype is not None and ctx.needs_input_grad[2]
+        fast = _lib.result(_lib.native().norm_backward(x2, w, dy, ctx.eps, need_w, need_b))
+        if fast is not None:
+            dx, dw, db = fast
+            return (dx, None if dw is None else dw.to(ctx.w_dtype), None if db is None else db.to(ctx.b_dtype), None)
+        x2 = x2.reshape(-1, x2.size(-1))
         rows, d = x2.shape
         dy2 = _rows(dy.to(x2.dtype))
         dx = torch.empty((rows, d), device=x2.device, dtype=x2.dtype)
-        need_w = ctx.w_dtype is not None and ctx.needs_input_grad[1]
-        need_b = ctx.b_dtype is not None and ctx.needs_input_grad[2]
         dw = torch.empty(d, device=x2.device, dtype=torch.float32) if need_w else None
         db = torch.empty(d, device=x2.device, dtype=torch.float32) if need_b else None
         x_in = x2 if (rows <= 1 or x2.stride(0) == d) else x2.contiguous()      # d_x is written with x's row pitch

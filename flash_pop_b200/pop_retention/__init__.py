@@ -22,8 +22,17 @@ class FlashPOPRetention(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, s, head_decays: Sequence[float], block_size: int, state_dtype: Optional[torch.dtype] = None):
-        head_decays = tuple(float(g) for g in head_decays)
         block_size = int(block_size)
+        if q.is_cuda and block_size > 0:
+            fast = _lib.result(_lib.native().forward(q, k, v, s, head_decays, state_dtype, _flags(), block_size))
+            if fast is not None:
+                sdt = fast[1].dtype
+                ctx.save_for_backward(q, k, v, s)
+                ctx.head_decays, ctx.block_size, ctx.state_dtype = head_decays, block_size, sdt
+                ctx.flags = _flags() | (_lib.FLAG_STATE_F32 if sdt != q.dtype else 0)
+                ctx.set_materialize_grads(False)
+                return fast
+        head_decays = tuple(float(g) for g in head_decays)
         q, k, v, s = _prepare(q, k, v, s, head_decays)
         B, T, H, dk = q.shape
         dv = v.shape[-1]
@@ -48,6 +57,12 @@ class FlashPOPRetention(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dO, d_block_states):
         q, k, v, s = ctx.saved_tensors
+        need = ctx.needs_input_grad
+        need_s = s is not None and need[3]
+        fast = _lib.result(_lib.native().backward(q, k, v, s, dO, d_block_states, ctx.head_decays, ctx.state_dtype, ctx.flags,
+                                                  ctx.block_size, need[0], need[1] or need[2] or need_s, need_s))
+        if fast is not None:
+            return *fast, None, None, None
         B, T, H, dk = q.shape
         dv = v.shape[-1]
         if dO is None:
@@ -104,6 +119,14 @@ class POPSuffixRetention(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, sq, sk, sv, s, block_states, head_decays: Sequence[float]):
+        if sq.is_cuda:
+            fast = _lib.result(_lib.native().suffix_forward(sq, sk, sv, s, block_states, head_decays, _flags()))
+            if fast is not None:
+                o, fq, fk, fv = fast
+                ctx.save_for_backward(fq, fk, fv, s, block_states)
+                ctx.head_decays, ctx.shape = head_decays, (*sq.shape[:2], block_states.shape[1])
+                ctx.flags = _flags() | (_lib.FLAG_STATE_F32 if block_states.dtype != sq.dtype else 0)
+                return o
         head_decays = tuple(float(g) for g in head_decays)
         _lib.require_cuda(sq, sk, sv, s, block_states)
         if sq.dim() != 5:
@@ -133,6 +156,9 @@ class POPSuffixRetention(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dO):
         fq, fk, fv, s, block_states = ctx.saved_tensors
+        fast = _lib.result(_lib.native().suffix_backward(fq, fk, fv, s, block_states, dO, ctx.head_decays, ctx.flags))
+        if fast is not None:
+            return *fast, None
         B, M, N = ctx.shape
         _, P, H, dk = fq.shape
         dv = fv.shape[-1]

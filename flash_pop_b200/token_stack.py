@@ -21,7 +21,6 @@ from flash_pop_b200.xpos_emb import XPos
 MAX_ROWS = 64
 _BF, _F32 = torch.bfloat16, torch.float32
 _ACTS = {F.silu: _lib.ACT_SWISH, F.gelu: _lib.ACT_GELU, F.relu: _lib.ACT_RELU}
-_PLAIN = (nn.Parameter, Tensor)
 
 
 def _global_hooks() -> bool:
@@ -36,14 +35,6 @@ def _watched() -> bool:
             or torch.compiler.is_compiling() or torch.jit.is_tracing() or _global_hooks())
 
 
-def _tensor(t, shape, dtype, device, align) -> int:
-    """Address of a parameter that the kernels can read in place; None when it is not one."""
-    if type(t) not in _PLAIN or t.dtype != dtype or t.shape != shape or t.device != device or not t.is_contiguous():
-        return None
-    ptr = t.data_ptr()
-    return None if ptr % align else ptr
-
-
 def _linear(m, n_out, n_in, device, out: list) -> bool:
     if type(m) is not nn.Linear:
         return False
@@ -51,13 +42,14 @@ def _linear(m, n_out, n_in, device, out: list) -> bool:
     if d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"] or "forward" in d:
         return False
     p = d["_parameters"]
-    w = _tensor(p.get("weight"), (n_out, n_in), _BF, device, 16)
+    address = _lib.native().address           # of a parameter that the kernels can read in place, or None
+    w = address(p.get("weight"), _BF, 16, device, n_out, n_in)
     if w is None:
         return False
     b = p.get("bias", d)                      # (a parametrised or deleted bias is not in the table at all)
     if b is d:
         return False
-    b = 0 if b is None else _tensor(b, (n_out,), _BF, device, 4)
+    b = 0 if b is None else address(b, _BF, 4, device, n_out, 0)
     if b is None:
         return False
     out += (w, b)
@@ -72,17 +64,17 @@ def _norm(m, width, device, out: list) -> bool:
         t = d.get(name, m)
         if t is m:
             return False
-        t = 0 if t is None else _tensor(t, (width,), _F32, device, 16)
+        t = 0 if t is None else _lib.native().address(t, _F32, 16, device, width, 0)
         if t is None:
             return False
         out.append(t)
     return True
 
 
-def _layer(layer, first, shape, device, index, layer_cls, retention_cls):
+def _layer(layer, first, shape, x_device, index, layer_cls, retention_cls):
     """(pointers, phasor address, tail of the layer's record) of a layer the kernels can run as it stands, else None."""
     H, dk, dv, ffn = shape
-    width = H * dv
+    width, device = H * dv, x_device.index
     cls, own = type(layer), layer.__dict__
     mods = own["_modules"]
     ret = mods["retention"]
@@ -118,7 +110,7 @@ def _layer(layer, first, shape, device, index, layer_cls, retention_cls):
         xpos = ret.xpos_embedder
         if type(xpos) is not XPos or xpos.head_dim != dk:
             return None
-        xpos._move(device)
+        xpos._move(x_device)
         row = xpos._rotation(1, index)
         ptrs.append(row.data_ptr())
     else:
