@@ -1,22 +1,26 @@
 // One token through a stack of decoder layers (flash_pop/retnet.py:181-199,247-268: pre-norm, retention step, gate, output
-// projection, feed-forward), five launches per layer, for batches of up to 64 rows:
-//   1. project_kernel   LayerNorm of the row, then the q, k, v and gate projections
-//   2. mix_kernel       rotation of q and k, S' = gamma S + k^T v / sqrt(dk), o = q S', GroupNorm of the head, gate
-//   3. project_kernel   output projection + residual
-//   4. project_kernel   LayerNorm, first feed-forward matrix, activation
-//   5. project_kernel   second feed-forward matrix + residual
+// projection, feed-forward) in one cooperative launch, for batches of up to 64 rows.  Per layer five phases, a grid
+// barrier after each:
+//   0. LayerNorm of the rows, then the q, k, v and gate projections
+//   1. rotation of q and k, S' = gamma S + k^T v / sqrt(dk), o = q S', GroupNorm of the head, gate
+//   2. output projection + residual
+//   3. LayerNorm, first feed-forward matrix, activation
+//   4. second feed-forward matrix + residual
 //
 // What bounds it.  A token reads every weight and every state once and does next to no arithmetic, so the floor is HBM:
-// 12 layers of d_model 1024, ffn 4096, 16 rows with fp32 states are 529 MB, 80 us at 6.65 TB/s.  As separate library and
-// elementwise launches (20 a layer) the stack took 942 us on the device and 5900 us on the host.  A launch of one matrix
-// is 1 to 8 MB, a microsecond of HBM time, so what counts is that every load of a launch is in flight at once and that no
-// launch waits for its predecessor before it starts loading:
-//   * a CTA owns NT weight rows over the whole contraction, its eight warps split K, and every warp requests its first
-//     16 KB-a-warp of weights (16 x 16 bytes a thread: all there is for K <= 4096) before anything else;
-//   * the launches are chained by programmatic dependent launch: weights and states, which no launch of the chain
-//     writes, are requested before griddepcontrol.wait, i.e. while the predecessor is still running.  A kernel lets its
-//     successor start only after its own wait, so whatever runs ahead of its wait has all launches but the last before
-//     it behind it; every kernel waits, so the last one's end is the end of all.
+// 12 layers of d_model 1024, ffn 4096, 16 rows with fp32 states are 529 MB, 80 us at 6.65 TB/s, a microsecond a phase.
+// What a phase costs beyond that is latency: of its first loads and of the hand-over from the phase before.  So
+//   * weights and states are requested into L2 two phases ahead, and every thread loads its first 128 bytes of the next
+//     phase's, with its bias and norm parameters, before it arrives at the barrier - no phase writes any of them - so HBM
+//     streams while the grid synchronises;
+//   * a phase deals its weight rows out in eights, evenly over the SMs, and the 16 warps of a CTA split the contraction;
+//   * up to 16 rows each CTA normalises the rows it reads itself, one warp a row; beyond, 128 KB of rows read and normalised
+//     by every SM cost more (38000 cycles at 64 rows) than a phase of its own that does it once.
+// Measured (12 layers as above, device time by graph replay / with the host work): 241 library and elementwise launches
+// 942 / 5870 us, five launches a layer chained by programmatic dependent launch 395 / 422 us, one launch 372 / 374 us (1 row
+// 332, 32 rows 489, 64 rows 801; the chained launches took 895 at 64).  A phase is 7000 to 13000 cycles, 2000 of them the
+// barrier; the rest is dependent round trips to L2 (700 to 1000 cycles each) and straight-line code run once.
+//
 // The products run on mma.sync.m16n8k16: rows of the batch x 8 weight rows, straight from the registers the 16-byte
 // loads fill (the contraction index is permuted the same way in both operands: thread t of a quad holds elements
 // 8t..8t+7 of every 32).  At 16 rows a weight byte feeds 16 multiply-adds, a hundredth of what tensor memory and
@@ -29,15 +33,35 @@ namespace fpb {
 namespace {
 
 typedef __nv_bfloat16 bf16;
-constexpr int THREADS = 256, WARPS = 8;
+constexpr int THREADS = 512, WARPS = 16;
 constexpr int MAX_B = 64, MAX_D = 1024;          // rows of a batch; channels of a LayerNorm row (4 x 8 a lane)
+constexpr int MAX_LAYERS = 16;                   // of a launch (the layers' records are kernel parameters)
+constexpr int PF = 8;                            // 16-byte pieces a thread has in flight
 
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+struct TokenParams {
+  int32_t B, H, dk, dv, ffn, layers, prev_f32, out_f32;
+  const bf16* x; int64_t x_stride;
+  bf16* y; int64_t y_stride;
+  bf16 *qkvg, *gated, *mid, *between, *hidden, *normed;   // (B, 2 H dk + 2 H dv), (B, H dv) three times, (B, ffn), (B, H dv)
+  unsigned* arrived;                              // the grid barrier's count, zero at the start
+  int32_t* status;
+  long long wait_cycles;
+  float gamma[FPB_MAX_HEADS];
+  fpb_decoder_layer layer[MAX_LAYERS];
+};
+
 __device__ __forceinline__ uint4 ld_stream(const void* p) {      // read once: keep it out of L1
   uint4 v;
   asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
+}
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void add_release(unsigned* p) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
 }
 __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -59,321 +83,519 @@ __device__ __forceinline__ float activate(int kind, float x) {
   if (kind == FPB_ACT_RELU) return x < 0.0f ? 0.0f : x;          // (NaN passes)
   return x;
 }
+// What other CTAs wrote during this launch is read past L1, which nothing keeps coherent.
+__device__ __forceinline__ uint4 ld_fresh(const void* p) { return __ldcg(reinterpret_cast<const uint4*>(p)); }
 
-struct ProjectParams {
-  const bf16* x; int64_t x_stride;               // (B, K) input rows
-  const float *norm_w, *norm_b; float eps;       // LayerNorm of the rows (NORM launches); either may be null
-  const bf16* w[4]; const bf16* bias[4];         // up to four (n_i, K) matrices whose outputs follow one another
-  int32_t n_end[4];                              // last output + 1 of each
-  const bf16* residual; int64_t res_stride;      // added to the (bf16-rounded) projection, or null
+// One projection phase: y = x W^T with up to four matrices whose outputs follow one another.  Kept in shared memory: made
+// anew from the kernel's parameters in every phase it cost 800 cycles each time (constant-cache misses).
+struct Job {
+  const void* w[4]; const void* bias[4];
+  int32_t n_beg[4], n_end[4];                     // first output of each and last + 1
+  int32_t N, K, act;
+  const float *norm_w, *norm_b; float eps;        // phases 0 and 3
+  const bf16* in; int64_t in_stride;              // rows that the norm reads
+  const bf16* x; int64_t x_stride;                // rows that the products read: the same, or their norms
+  const bf16* residual; int64_t res_stride;
   bf16* y; int64_t y_stride;
-  int32_t B, K, act;
 };
 
-__host__ __device__ constexpr int norm_pitch(int K) { return K * 2 + 64; }   // bytes: eight rows x four 16-byte pieces of a quad tile all 32 banks
+__host__ __device__ constexpr int norm_pitch(int K) { return K * 2 + 64; }   // bytes: eight rows x a quad's pieces tile all banks
 
-// N8: weight rows a CTA owns / 8; MT: batch rows / 16, rounded up.
-template <int N8, int MT, bool NORM>
-__global__ void __launch_bounds__(THREADS, MT <= 2 ? 2 : 1) project_kernel(const __grid_constant__ ProjectParams p) {
-  constexpr int NT = N8 * 8, BLK = 16 / N8;      // BLK: 32-wide contraction steps whose weights are in flight together
-  extern __shared__ __align__(16) uint8_t sm[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int n0 = blockIdx.x * NT;
+__device__ __forceinline__ Job job_of(const TokenParams& p, int i, int phase, bool normed) {
+  const fpb_decoder_layer& l = p.layer[i];
+  const int width = p.H * p.dv, qk = p.H * p.dk;
+  const bf16* in = i == 0 ? p.x : p.between;
+  const int64_t in_stride = i == 0 ? p.x_stride : width;
+  Job j{};
+  j.act = FPB_ACT_NONE;
+  if (phase == 0) {
+    j.w[0] = l.wq; j.w[1] = l.wk; j.w[2] = l.wv; j.w[3] = l.wg;
+    j.bias[0] = l.bq; j.bias[1] = l.bk; j.bias[2] = l.bv; j.bias[3] = l.bg;
+    j.n_end[0] = qk; j.n_end[1] = 2 * qk; j.n_end[2] = 2 * qk + width; j.n_end[3] = 2 * qk + 2 * width;
+    j.K = width; j.norm_w = l.norm1_w; j.norm_b = l.norm1_b; j.eps = (float)l.norm1_eps;
+    j.x = in; j.x_stride = in_stride; j.y = p.qkvg; j.y_stride = j.n_end[3];
+  } else {
+    j.w[0] = phase == 2 ? l.wo : phase == 3 ? l.w1 : l.w2;
+    j.bias[0] = phase == 2 ? l.bo : phase == 3 ? l.b1 : l.b2;
+    const int n = phase == 3 ? p.ffn : width;
+    j.n_end[0] = j.n_end[1] = j.n_end[2] = j.n_end[3] = n;
+    j.K = phase == 4 ? p.ffn : width;
+    j.x = phase == 2 ? p.gated : phase == 3 ? p.mid : p.hidden; j.x_stride = j.K;
+    j.y = phase == 2 ? p.mid : phase == 3 ? p.hidden : p.between; j.y_stride = n;
+    if (phase == 2) { j.residual = in; j.res_stride = in_stride; }
+    if (phase == 3) { j.norm_w = l.norm2_w; j.norm_b = l.norm2_b; j.eps = (float)l.norm2_eps; j.act = (int)l.act_ffn; }
+    if (phase == 4) {
+      j.residual = p.mid; j.res_stride = width;
+      if (i == p.layers - 1) { j.y = p.y; j.y_stride = p.y_stride; }
+    }
+  }
+  j.in = j.x; j.in_stride = j.x_stride;
+  if (normed && (phase == 0 || phase == 3)) { j.x = p.normed; j.x_stride = width; }
+  j.n_beg[0] = 0; j.n_beg[1] = j.n_end[0]; j.n_beg[2] = j.n_end[1]; j.n_beg[3] = j.n_end[2];
+  j.N = j.n_end[3];
+  return j;
+}
+
+struct Share { int c0, c1, k0, k1; };             // weight rows / 8 of this CTA; 32-wide contraction steps of this warp
+__device__ __forceinline__ Share share_of(const Job& j, const int2& tiles) {
+  const int steps = j.K >> 5, warp = threadIdx.x >> 5;
+  return {tiles.x, tiles.y, steps * warp / WARPS, steps * (warp + 1) / WARPS};
+}
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void copy_async16(void* smem, const void* p) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(p) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ int matrix_of(const Job& j, int n0) {
   int m = 0;
 #pragma unroll
-  for (int i = 0; i < 3; ++i) m += n0 >= p.n_end[i] ? 1 : 0;
-  const int n_first = n0 - (m ? p.n_end[m - 1] : 0);
-  const int K = p.K, steps = K >> 5;
-  const int i0 = steps * warp / WARPS, i1 = steps * (warp + 1) / WARPS;
-  const bf16* w = p.w[m] + (int64_t)(n_first + g) * K + t * 8;
+  for (int i = 0; i < 3; ++i) m += n0 >= j.n_end[i] ? 1 : 0;
+  return m;
+}
+// this thread's pieces of weight tiles [tile, tile + TPP), steps [step, step + PF / TPP)
+template <int TPP> __device__ __forceinline__ void fetch_weights(uint4 (&w)[PF], const Job& j, const Share& s, int tile, int step) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int c = 0; c < TPP; ++c) {
+    const int n0 = (tile + c) * 8, m = matrix_of(j, n0);
+    const bf16* base = (const bf16*)j.w[m] + (int64_t)(n0 - j.n_beg[m] + g) * j.K + t * 8;
+#pragma unroll
+    for (int i = 0; i < PF / TPP; ++i)
+      if (tile + c < s.c1 && step + i < s.k1) w[i * TPP + c] = ld_stream(base + (step + i) * 32);
+  }
+}
 
-  uint4 wr[BLK][N8];
-  auto fetch = [&](int base) {
+// the bias of the column pair this thread finishes
+template <int TPP> __device__ __forceinline__ uint32_t fetch_bias(const Job& j, const Share& s, int tile) {
+  const int n = tile * 8 + (threadIdx.x % (TPP * 4)) * 2, m = matrix_of(j, n);
+  const bf16* bias = (const bf16*)j.bias[m];
+  return bias && n < s.c1 * 8 ? __ldg(reinterpret_cast<const unsigned*>(bias + n - j.n_beg[m])) : 0u;
+}
+
+// the norm's weight and bias, MAX_D floats each, into shared memory ahead of the barrier
+__device__ __forceinline__ void stage_norm(float* dst, const Job& j) {
+  const int i = (threadIdx.x & 255) * 4;
+  const float* src = threadIdx.x < 256 ? j.norm_w : j.norm_b;
+  float* to = dst + (threadIdx.x < 256 ? 0 : MAX_D) + i;
+  if (i >= j.K) return;
+  const float fill = threadIdx.x < 256 ? 1.0f : 0.0f;
+  if (src) copy_async16(to, src + i);
+  else *reinterpret_cast<float4*>(to) = make_float4(fill, fill, fill, fill);
+}
+static_assert(THREADS == 512 && MAX_D == 1024, "one 16-byte piece a thread");
+
+// LayerNorm of the batch's rows, rounded to bf16 as the operand of the products: a warp a row, its next row on its way.  Four channels a lane and piece: the parameters' 16-byte loads then meet no bank conflict.
+__device__ __forceinline__ void normalise(uint8_t* to, int64_t pitch, const float* norm, const Job& j, int first, int stride, int B) {
+  constexpr int NP = MAX_D / 128;
+  const int lane = threadIdx.x & 31, K = j.K;
+  const float inv = 1.0f / (float)K, eps = j.eps;
+  uint2 in[NP];
+  auto request = [&](int row) {
 #pragma unroll
-    for (int j = 0; j < BLK; ++j)
-#pragma unroll
-      for (int c = 0; c < N8; ++c)
-        if (base + j < i1) wr[j][c] = ld_stream(w + (int64_t)c * 8 * K + (base + j) * 32);
+    for (int i = 0; i < NP; ++i)
+      if (row < B && 4 * (lane + 32 * i) < K) in[i] = __ldcg(reinterpret_cast<const uint2*>(j.in + row * j.in_stride + 4 * (lane + 32 * i)));
   };
-  fetch(i0);
-  grid_wait();
-  grid_release();
-
-  const int pitch = norm_pitch(K);
-  if constexpr (NORM) {                           // normalised rows, rounded to bf16 as the operand of the products
-    for (int row = warp; row < p.B; row += WARPS) {
-      const bf16* x = p.x + row * p.x_stride;
-      float f[4][8];
-      float sum = 0.0f;
+  request(first);
+  for (int row = first; row < B; row += stride) {
+    float f[NP][4];
+    float sum = 0.0f;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int c = 8 * (lane + 32 * i);
-        if (c < K) {
-          const uint4 raw = *reinterpret_cast<const uint4*>(x + c);
-          const uint32_t e[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-          for (int j = 0; j < 4; ++j) { const float2 a = unpack2(e[j]); f[i][2 * j] = a.x; f[i][2 * j + 1] = a.y; sum += a.x + a.y; }
-        }
-      }
-      const float mean = warp_sum(sum) / (float)K;
-      float sq = 0.0f;
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (8 * (lane + 32 * i) < K) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) { f[i][j] -= mean; sq += f[i][j] * f[i][j]; }
-        }
-      const float rstd = rsqrtf(warp_sum(sq) / (float)K + p.eps);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int c = 8 * (lane + 32 * i);
-        if (c < K) {
-          uint32_t e[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float2 gw = p.norm_w ? __ldg(reinterpret_cast<const float2*>(p.norm_w + c) + j) : make_float2(1.0f, 1.0f);
-            const float2 gb = p.norm_b ? __ldg(reinterpret_cast<const float2*>(p.norm_b + c) + j) : make_float2(0.0f, 0.0f);
-            e[j] = pack2(f[i][2 * j] * rstd * gw.x + gb.x, f[i][2 * j + 1] * rstd * gw.y + gb.y);
-          }
-          *reinterpret_cast<uint4*>(sm + row * pitch + c * 2) = make_uint4(e[0], e[1], e[2], e[3]);
-        }
+    for (int i = 0; i < NP; ++i) {
+      if (4 * (lane + 32 * i) < K) {
+        const float2 a = unpack2(in[i].x), b = unpack2(in[i].y);
+        f[i][0] = a.x; f[i][1] = a.y; f[i][2] = b.x; f[i][3] = b.y;
+        sum += (a.x + a.y) + (b.x + b.y);
       }
     }
-    __syncthreads();
+    request(row + stride);
+    const float mean = warp_sum(sum) * inv;
+    float sq = 0.0f;
+#pragma unroll
+    for (int i = 0; i < NP; ++i)
+      if (4 * (lane + 32 * i) < K) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { f[i][k] -= mean; sq += f[i][k] * f[i][k]; }
+      }
+    const float rstd = rsqrtf(warp_sum(sq) * inv + eps);
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      const int c = 4 * (lane + 32 * i);
+      if (c < K) {
+        const float4 gw = *reinterpret_cast<const float4*>(norm + c), gb = *reinterpret_cast<const float4*>(norm + MAX_D + c);
+        *reinterpret_cast<uint2*>(to + row * pitch + c * 2) = make_uint2(pack2(f[i][0] * rstd * gw.x + gb.x, f[i][1] * rstd * gw.y + gb.y),
+                                                                         pack2(f[i][2] * rstd * gw.z + gb.z, f[i][3] * rstd * gw.w + gb.w));
+      }
+    }
   }
+}
 
-  float acc[MT][N8][4];
-#pragma unroll
-  for (int a = 0; a < MT; ++a)
-#pragma unroll
-    for (int c = 0; c < N8; ++c)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[a][c][e] = 0.0f;
+// The products of this CTA's weight rows, TPP tiles of eight at a time.  w holds the first pieces on entry.
+template <int MT, int TPP, bool NORM>
+__device__ __forceinline__ void project(uint8_t* sm, uint4 (&w)[PF], uint32_t bias, const Job& j, const Share& s, int B) {
+  constexpr int STEPS = PF / TPP, RP = TPP * 8 + 2;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, pitch = norm_pitch(j.K);
+  float* red = reinterpret_cast<float*>(sm + (NORM ? MT * 16 * pitch : 0));      // [WARPS][MT * 16][RP]
   // rows past the batch repeat its last row; their sums are dropped
   auto x_piece = [&](int row, int step) -> uint4 {
-    row = min(row, p.B - 1);
+    row = min(row, B - 1);
     if constexpr (NORM) return *reinterpret_cast<const uint4*>(sm + row * pitch + (step * 32 + t * 8) * 2);
-    else return *reinterpret_cast<const uint4*>(p.x + row * p.x_stride + step * 32 + t * 8);
+    else return ld_fresh(j.x + row * j.x_stride + step * 32 + t * 8);
   };
-  constexpr int XB = MT == 1 ? 4 : MT == 2 ? 2 : 1;        // steps whose inputs are in flight together
-  for (int base = i0; base < i1; base += BLK) {
+  constexpr int XB = MT == 1 ? (STEPS < 4 ? STEPS : 4) : MT == 2 ? (STEPS < 2 ? STEPS : 2) : 1;   // steps whose inputs are in flight together
+  const int c_own = (threadIdx.x % (TPP * 4)) * 2;           // the column pair this thread finishes, in every row it takes
+  for (int tile = s.c0; tile < s.c1; tile += TPP) {
+    if (tile > s.c0) bias = fetch_bias<TPP>(j, s, tile);
+    uint32_t res = 0;                                        // (written two phases ago or earlier)
+    const int n_own = tile * 8 + c_own, row_own = threadIdx.x / (TPP * 4);
+    if (j.residual && row_own < B && n_own < s.c1 * 8) res = __ldcg(reinterpret_cast<const unsigned*>(j.residual + row_own * j.res_stride + n_own));
+    float acc[MT][TPP][4];
 #pragma unroll
-    for (int j0 = 0; j0 < BLK; j0 += XB) {
-      uint4 lo[XB][MT], hi[XB][MT];
+    for (int a = 0; a < MT; ++a)
 #pragma unroll
-      for (int j = 0; j < XB; ++j)
+      for (int c = 0; c < TPP; ++c)
 #pragma unroll
-        for (int a = 0; a < MT; ++a) {
-          const int step = min(base + j0 + j, i1 - 1);
-          lo[j][a] = x_piece(a * 16 + g, step);
-          hi[j][a] = x_piece(a * 16 + g + 8, step);
-        }
+        for (int e = 0; e < 4; ++e) acc[a][c][e] = 0.0f;
+    for (int base = s.k0; base < s.k1; base += STEPS) {
+      if (tile > s.c0 || base > s.k0) fetch_weights<TPP>(w, j, s, tile, base);
 #pragma unroll
-      for (int j = 0; j < XB; ++j) {
-        if (base + j0 + j >= i1) break;
+      for (int i0 = 0; i0 < STEPS; i0 += XB) {
+        uint4 lo[XB][MT], hi[XB][MT];
 #pragma unroll
-        for (int a = 0; a < MT; ++a)
+        for (int i = 0; i < XB; ++i)
 #pragma unroll
-          for (int c = 0; c < N8; ++c) {
-            const uint4 b = wr[j0 + j][c];
-            mma_16816(acc[a][c], lo[j][a].x, hi[j][a].x, lo[j][a].y, hi[j][a].y, b.x, b.y);
-            mma_16816(acc[a][c], lo[j][a].z, hi[j][a].z, lo[j][a].w, hi[j][a].w, b.z, b.w);
+          for (int a = 0; a < MT; ++a) {
+            const int step = min(base + i0 + i, s.k1 - 1);
+            lo[i][a] = x_piece(a * 16 + g, step);
+            hi[i][a] = x_piece(a * 16 + g + 8, step);
           }
+#pragma unroll
+        for (int i = 0; i < XB; ++i) {
+          if (base + i0 + i >= s.k1) break;
+#pragma unroll
+          for (int a = 0; a < MT; ++a)
+#pragma unroll
+            for (int c = 0; c < TPP; ++c) {
+              const uint4 b = w[(i0 + i) * TPP + c];         // (tiles past the CTA's share: stale, their sums are dropped)
+              mma_16816(acc[a][c], lo[i][a].x, hi[i][a].x, lo[i][a].y, hi[i][a].y, b.x, b.y);
+              mma_16816(acc[a][c], lo[i][a].z, hi[i][a].z, lo[i][a].w, hi[i][a].w, b.z, b.w);
+            }
+        }
       }
     }
-    fetch(base + BLK);
-  }
-
-  // the warps' partial sums over K
-  float* red = reinterpret_cast<float*>(sm + (NORM ? MT * 16 * pitch : 0));   // [WARPS][MT * 16][NT + 2]
-  constexpr int RP = NT + 2;
 #pragma unroll
-  for (int a = 0; a < MT; ++a)
+    for (int a = 0; a < MT; ++a)
 #pragma unroll
-    for (int c = 0; c < N8; ++c) {
-      float* r = red + ((warp * MT + a) * 16 + g) * RP + c * 8 + 2 * t;
-      *reinterpret_cast<float2*>(r) = make_float2(acc[a][c][0], acc[a][c][1]);
-      *reinterpret_cast<float2*>(r + 8 * RP) = make_float2(acc[a][c][2], acc[a][c][3]);
-    }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < p.B * (NT / 2); idx += THREADS) {
-    const int row = idx / (NT / 2), c = (idx % (NT / 2)) * 2;
-    float2 s = make_float2(0.0f, 0.0f);
+      for (int c = 0; c < TPP; ++c) {
+        float* r = red + ((warp * MT + a) * 16 + g) * RP + c * 8 + 2 * t;
+        *reinterpret_cast<float2*>(r) = make_float2(acc[a][c][0], acc[a][c][1]);
+        *reinterpret_cast<float2*>(r + 8 * RP) = make_float2(acc[a][c][2], acc[a][c][3]);
+      }
+    __syncthreads();
+    if (n_own < s.c1 * 8) {
+      const float2 b = unpack2(bias);
+      for (int row = row_own; row < B; row += THREADS / (TPP * 4)) {
+        float2 v = make_float2(0.0f, 0.0f);
 #pragma unroll
-    for (int k = 0; k < WARPS; ++k) {
-      const float2 v = *reinterpret_cast<const float2*>(red + (k * MT * 16 + row) * RP + c);
-      s.x += v.x; s.y += v.y;
+        for (int k = 0; k < WARPS; ++k) {
+          const float2 f = *reinterpret_cast<const float2*>(red + (k * MT * 16 + row) * RP + c_own);
+          v.x += f.x; v.y += f.y;
+        }
+        v.x = activate(j.act, v.x + b.x); v.y = activate(j.act, v.y + b.y);
+        uint32_t out = pack2(v.x, v.y);
+        if (j.residual) {
+          if (row != row_own) res = __ldcg(reinterpret_cast<const unsigned*>(j.residual + row * j.res_stride + n_own));
+          const float2 f = unpack2(out), r = unpack2(res);
+          out = pack2(r.x + f.x, r.y + f.y);
+        }
+        *reinterpret_cast<uint32_t*>(j.y + row * j.y_stride + n_own) = out;
+      }
     }
-    if (p.bias[m]) {
-      const float2 b = unpack2(*reinterpret_cast<const uint32_t*>(p.bias[m] + n_first + c));
-      s.x += b.x; s.y += b.y;
-    }
-    s.x = activate(p.act, s.x); s.y = activate(p.act, s.y);
-    uint32_t out = pack2(s.x, s.y);
-    if (p.residual) {
-      const float2 y = unpack2(out), r = unpack2(*reinterpret_cast<const uint32_t*>(p.residual + row * p.res_stride + n0 + c));
-      out = pack2(r.x + y.x, r.y + y.y);
-    }
-    *reinterpret_cast<uint32_t*>(p.y + row * p.y_stride + n0 + c) = out;
+    __syncthreads();                              // (the sums are overwritten by the next tiles, or the next phase)
   }
 }
 
-struct MixParams {
-  const bf16* qkvg;                               // (B, 2 H dk + 2 H dv): q | k | v | gate
-  const float2* phasors;                          // (dk / 2) of (cos, sin) for this position, or null
-  const void* s_prev; int64_t prev_sb, prev_sh;   // null: a zero state
-  void* s_out; int64_t out_sb, out_sh;
-  bf16* y;                                        // (B, H dv)
-  int32_t H, dk, dv, act;
-  float gn_eps;
-  float gamma[FPB_MAX_HEADS];
+// ---- phase 1: a group of 512, 256 or 128 threads takes (row, head) after (row, head) - as many groups as there are heads for
+// an SM, one after another each costs 8000 cycles of latency; dv / 4 threads across the state's columns, PF passes of rows
+// in flight
+struct MixShape {
+  int threads, group, tid, first, stride;         // of the group; its first (row, head) and the step to its next
+  int ty_n, col, ty; bool live;
+  __device__ __forceinline__ explicit MixShape(const TokenParams& p) {
+    const int per_sm = (p.B * p.H + gridDim.x - 1) / gridDim.x, tx_n = p.dv >> 2;
+    threads = per_sm <= 1 ? THREADS : per_sm == 2 ? THREADS / 2 : THREADS / 4;
+    group = threadIdx.x / threads; tid = threadIdx.x % threads;
+    first = blockIdx.x + group * gridDim.x; stride = gridDim.x * (THREADS / threads);
+    ty_n = threads / tx_n; col = (tid % tx_n) * 4; ty = tid / tx_n; live = ty < ty_n;
+  }
+  __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(threads) : "memory"); }
 };
-
-template <typename T> __device__ __forceinline__ float4 load4(const T* p);
-template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
-template <> __device__ __forceinline__ float4 load4<bf16>(const bf16* p) {
-  const uint2 r = *reinterpret_cast<const uint2*>(p);
-  const float2 a = unpack2(r.x), b = unpack2(r.y);
-  return make_float4(a.x, a.y, b.x, b.y);
-}
-template <typename T> __device__ __forceinline__ void store4(T* p, float4 v);
-template <> __device__ __forceinline__ void store4<float>(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-template <> __device__ __forceinline__ void store4<bf16>(bf16* p, float4 v) { *reinterpret_cast<uint2*>(p) = make_uint2(pack2(v.x, v.y), pack2(v.z, v.w)); }
-
-// A CTA owns one (row, head): dv / 4 threads across the state's columns, as many rows at a time as the 256 threads hold,
-// eight passes of rows in flight while the eight before them are worked on.
-template <typename TP, typename TO>
-__global__ void __launch_bounds__(THREADS, 2) mix_kernel(const __grid_constant__ MixParams p) {
-  constexpr int UN = 8;
-  __shared__ float sh_q[256], sh_k[256], sh_red[2][WARPS];
-  __shared__ float sh_o[THREADS * 4];
-  const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
-  const int tx_n = p.dv >> 2, ty_n = THREADS / tx_n;
-  const int tx = tid % tx_n, ty = tid / tx_n, col = tx * 4;
-  const bool live = ty < ty_n;
-  const TP* sp = p.s_prev && live ? (const TP*)p.s_prev + b * p.prev_sb + h * p.prev_sh + col : nullptr;
-  TO* so = (TO*)p.s_out + b * p.out_sb + h * p.out_sh + col;
-  const float gamma = p.gamma[h];
-
-  float4 ra[UN], rb[UN];
-  auto fetch = [&](float4 (&r)[UN], int r0) {
+__device__ __forceinline__ void fetch_state(uint4 (&r)[PF], const TokenParams& p, const fpb_decoder_layer& l, const MixShape& m, int unit, int row0) {
+  const int64_t at = (unit / p.H) * l.prev_sb + (unit % p.H) * l.prev_sh + m.col;
 #pragma unroll
-    for (int u = 0; u < UN; ++u) {
-      const int row = r0 + u * ty_n;
-      r[u] = sp && row < p.dk ? load4<TP>(sp + (int64_t)row * p.dv) : make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int u = 0; u < PF; ++u) {
+    const int row = row0 + u * m.ty_n;
+    r[u] = make_uint4(0u, 0u, 0u, 0u);
+    if (!l.s_prev || !m.live || row >= p.dk || unit >= p.B * p.H) continue;
+    if (p.prev_f32) r[u] = ld_stream((const float*)l.s_prev + at + (int64_t)row * p.dv);
+    else {
+      const uint2 v = __ldg(reinterpret_cast<const uint2*>((const bf16*)l.s_prev + at + (int64_t)row * p.dv));
+      const float2 a = unpack2(v.x), b = unpack2(v.y);
+      r[u] = make_uint4(__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(b.x), __float_as_uint(b.y));
     }
-  };
-  fetch(ra, ty);
-  grid_wait();
-  grid_release();
-
-  const int qk = p.H * p.dk, width = p.H * p.dv;
-  const bf16* in = p.qkvg + (int64_t)b * (2 * qk + 2 * width);
-  const float rs = rsqrtf((float)p.dk);
-  for (int i = tid; i < p.dk / 2; i += THREADS) {
-    float2 q = unpack2(*reinterpret_cast<const uint32_t*>(in + h * p.dk + 2 * i));
-    float2 k = unpack2(*reinterpret_cast<const uint32_t*>(in + qk + h * p.dk + 2 * i));
-    if (p.phasors) {
-      const float2 c = p.phasors[i];
-      q = make_float2(q.x * c.x - q.y * c.y, q.x * c.y + q.y * c.x);
-      k = make_float2(k.x * c.x - k.y * c.y, k.x * c.y + k.y * c.x);
-    }
-    sh_q[2 * i] = q.x; sh_q[2 * i + 1] = q.y;
-    sh_k[2 * i] = k.x * rs; sh_k[2 * i + 1] = k.y * rs;
   }
-  const float4 v = live ? load4<bf16>(in + 2 * qk + h * p.dv + col) : make_float4(0.f, 0.f, 0.f, 0.f);
-  const float z = tid < p.dv ? __bfloat162float(in[2 * qk + width + h * p.dv + tid]) : 0.0f;
-  __syncthreads();
-  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-  auto update = [&](const float4 (&r)[UN], int r0) {
+}
+__device__ __forceinline__ void mix(float* sh, uint4 (&r)[PF], const TokenParams& p, const fpb_decoder_layer& l) {
+  const MixShape m(p);
+  float *sh_q = sh + m.group * 512, *sh_k = sh_q + 256, *sh_o = sh + 2048 + m.group * m.threads * 4;
+  const int tid = m.tid, qk = p.H * p.dk, width = p.H * p.dv, pass = PF * m.ty_n;
+  const float rs = rsqrtf((float)p.dk);
+  for (int unit = m.first; unit < p.B * p.H; unit += m.stride) {
+    const int b = unit / p.H, h = unit % p.H;
+    const float gamma = p.gamma[h];
+    const bf16* in = p.qkvg + (int64_t)b * (2 * qk + 2 * width);
+    for (int i = tid; i < p.dk / 2; i += m.threads) {
+      float2 q = unpack2(__ldcg(reinterpret_cast<const unsigned*>(in + h * p.dk + 2 * i)));
+      float2 k = unpack2(__ldcg(reinterpret_cast<const unsigned*>(in + qk + h * p.dk + 2 * i)));
+      if (l.phasors) {
+        const float2 c = __ldg(reinterpret_cast<const float2*>(l.phasors) + i);
+        q = make_float2(q.x * c.x - q.y * c.y, q.x * c.y + q.y * c.x);
+        k = make_float2(k.x * c.x - k.y * c.y, k.x * c.y + k.y * c.x);
+      }
+      sh_q[2 * i] = q.x; sh_q[2 * i + 1] = q.y;
+      sh_k[2 * i] = k.x * rs; sh_k[2 * i + 1] = k.y * rs;
+    }
+    float2 v01 = make_float2(0.f, 0.f), v23 = v01;
+    if (m.live) {
+      const uint2 v = __ldcg(reinterpret_cast<const uint2*>(in + 2 * qk + h * p.dv + m.col));
+      v01 = unpack2(v.x); v23 = unpack2(v.y);
+    }
+    // GroupNorm and gate of the head: warp 0, channels 4 lane + 128 k
+    float2 z[2][2];
 #pragma unroll
-    for (int u = 0; u < UN; ++u) {
-      const int row = r0 + u * ty_n;
-      if (live && row < p.dk) {
+    for (int k = 0; k < 2; ++k) {
+      const int c = 4 * tid + 128 * k;
+      if (tid < 32 && c < p.dv) {
+        const uint2 v = __ldcg(reinterpret_cast<const uint2*>(in + 2 * qk + width + h * p.dv + c));
+        z[k][0] = unpack2(v.x); z[k][1] = unpack2(v.y);
+      }
+    }
+    m.sync();
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int64_t at = b * l.out_sb + h * l.out_sh + m.col;
+    for (int r0 = m.ty; r0 < p.dk; r0 += pass) {
+      if (r0 != m.ty) fetch_state(r, p, l, m, unit, r0);
+#pragma unroll
+      for (int u = 0; u < PF; ++u) {
+        const int row = r0 + u * m.ty_n;
+        if (!m.live || row >= p.dk) continue;
         const float kr = sh_k[row], qr = sh_q[row];
         float4 s;
-        s.x = fmaf(gamma, r[u].x, kr * v.x); s.y = fmaf(gamma, r[u].y, kr * v.y);
-        s.z = fmaf(gamma, r[u].z, kr * v.z); s.w = fmaf(gamma, r[u].w, kr * v.w);
+        s.x = fmaf(gamma, __uint_as_float(r[u].x), kr * v01.x); s.y = fmaf(gamma, __uint_as_float(r[u].y), kr * v01.y);
+        s.z = fmaf(gamma, __uint_as_float(r[u].z), kr * v23.x); s.w = fmaf(gamma, __uint_as_float(r[u].w), kr * v23.y);
         o.x = fmaf(qr, s.x, o.x); o.y = fmaf(qr, s.y, o.y); o.z = fmaf(qr, s.z, o.z); o.w = fmaf(qr, s.w, o.w);
-        store4<TO>(so + (int64_t)row * p.dv, s);
+        if (p.out_f32) *reinterpret_cast<float4*>((float*)l.s_out + at + (int64_t)row * p.dv) = s;
+        else *reinterpret_cast<uint2*>((bf16*)l.s_out + at + (int64_t)row * p.dv) = make_uint2(pack2(s.x, s.y), pack2(s.z, s.w));
+      }
+    }
+    if (unit + m.stride < p.B * p.H) fetch_state(r, p, l, m, unit + m.stride, m.ty);
+    if (m.live) *reinterpret_cast<float4*>(sh_o + m.ty * p.dv + m.col) = o;
+    m.sync();
+    // (the other warps go on to the next head: its q and k have buffers of their own to wait for only at the barrier above)
+    if (tid < 32) {
+      float x[2][4];
+      float sum = 0.0f;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int c = 4 * tid + 128 * k;
+        x[k][0] = x[k][1] = x[k][2] = x[k][3] = 0.0f;
+        if (c < p.dv)
+          for (int y = 0; y < m.ty_n; ++y) {
+            const float4 f = *reinterpret_cast<const float4*>(sh_o + y * p.dv + c);
+            x[k][0] += f.x; x[k][1] += f.y; x[k][2] += f.z; x[k][3] += f.w;
+          }
+        sum += (x[k][0] + x[k][1]) + (x[k][2] + x[k][3]);
+      }
+      const float mean = warp_sum(sum) / (float)p.dv;
+      float sq = 0.0f;
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        if (4 * tid + 128 * k < p.dv) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) { x[k][e] -= mean; sq += x[k][e] * x[k][e]; }
+        }
+      const float rstd = rsqrtf(warp_sum(sq) / (float)p.dv + (float)l.gn_eps);
+      const int act = (int)l.act_gate;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int c = 4 * tid + 128 * k;
+        if (c < p.dv)
+          *reinterpret_cast<uint2*>(p.gated + (int64_t)b * width + h * p.dv + c) =
+              make_uint2(pack2(x[k][0] * rstd * activate(act, z[k][0].x), x[k][1] * rstd * activate(act, z[k][0].y)),
+                         pack2(x[k][2] * rstd * activate(act, z[k][1].x), x[k][3] * rstd * activate(act, z[k][1].y)));
+      }
+    }
+  }
+}
+
+template <int MT, bool NORM>
+__device__ __forceinline__ void project_any(uint8_t* sm, uint4 (&w)[PF], uint32_t bias, const Job& j, const Share& s, int B) {
+  const int n = s.c1 - s.c0;
+  if (n <= 1) project<MT, 1, NORM>(sm, w, bias, j, s, B);
+  else if (n <= 2 || MT > 2) project<MT, 2, NORM>(sm, w, bias, j, s, B);
+  else if constexpr (MT <= 2) project<MT, 4, NORM>(sm, w, bias, j, s, B);
+}
+template <int MT> __device__ __forceinline__ void prefetch(uint4 (&w)[PF], uint32_t& bias, const Job& j, const Share& s) {
+  const int n = s.c1 - s.c0;
+  if (n <= 1) { fetch_weights<1>(w, j, s, s.c0, s.k0); bias = fetch_bias<1>(j, s, s.c0); }
+  else if (n <= 2 || MT > 2) { fetch_weights<2>(w, j, s, s.c0, s.k0); bias = fetch_bias<2>(j, s, s.c0); }
+  else if constexpr (MT <= 2) { fetch_weights<4>(w, j, s, s.c0, s.k0); bias = fetch_bias<4>(j, s, s.c0); }
+}
+
+constexpr int NORM_BYTES = 2 * MAX_D * 4;         // staged norm parameters, ahead of the phases' own shared memory
+
+// MT: batch rows / 16, rounded up
+template <int MT>
+__global__ void __launch_bounds__(THREADS, 1) token_kernel(const __grid_constant__ TokenParams p) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ int quit;
+  __shared__ int2 tiles[5];                       // this CTA's share of each phase's weight rows / 8
+  __shared__ Job jobs[2][5];                      // of this layer and the next ([1] is not used: no projection)
+  float* norm = reinterpret_cast<float*>(smem);
+  uint8_t* sm = smem + NORM_BYTES;
+  uint4 w[PF];
+  uint32_t bias = 0;
+  unsigned passed = 0;
+  if (threadIdx.x < 5) {
+    const int width = p.H * p.dv, n = threadIdx.x == 0 ? 2 * p.H * p.dk + 2 * width : threadIdx.x == 3 ? p.ffn : width;
+    const int64_t t = n >> 3, c = blockIdx.x, g = gridDim.x;
+    tiles[threadIdx.x] = make_int2((int)(t * c / g), (int)(t * (c + 1) / g));
+  }
+  auto make_jobs = [&](int i) {                   // one warp, a phase a lane
+    const int phase = threadIdx.x & 31;
+    if (i < p.layers && phase < 5 && phase != 1) jobs[i & 1][phase] = job_of(p, i, phase, MT > 1);
+  };
+  if (threadIdx.x < 32) { make_jobs(0); make_jobs(1); }
+  __syncthreads();
+  // Into L2 two phases ahead, so that HBM streams all the time and the register prefetch at the end of a phase is short:
+  // one bulk request a weight tile (eight rows) or state.
+  auto request_l2 = [&](int i, int phase) {
+    if (phase >= 5) { phase -= 5; ++i; }
+    if (i >= p.layers || threadIdx.x >= 32) return;
+    if (phase == 1) {
+      const fpb_decoder_layer& l = p.layer[i];
+      if (!l.s_prev) return;
+      const int esize = p.prev_f32 ? 4 : 2, bytes = p.dk * p.dv * esize;
+      for (int u = blockIdx.x + gridDim.x * threadIdx.x; u < p.B * p.H; u += gridDim.x * 32) {
+        const char* at = (const char*)l.s_prev + ((u / p.H) * l.prev_sb + (u % p.H) * l.prev_sh) * esize;
+        if (((uintptr_t)at | bytes) % 16 == 0) prefetch_l2(at, bytes);
+      }
+    } else {
+      const Job& j = jobs[i & 1][phase];
+      const int2 c = tiles[phase];
+      for (int tile = c.x + threadIdx.x; tile < c.y; tile += 32) {
+        const int m = matrix_of(j, tile * 8);
+        prefetch_l2((const bf16*)j.w[m] + (int64_t)(tile * 8 - j.n_beg[m]) * j.K, 8 * j.K * 2);
       }
     }
   };
-  const int pass = UN * ty_n;
-  for (int r0 = ty; r0 < p.dk; r0 += 2 * pass) {
-    fetch(rb, r0 + pass);
-    update(ra, r0);
-    fetch(ra, r0 + 2 * pass);
-    update(rb, r0 + pass);
-  }
-  if (live) *reinterpret_cast<float4*>(sh_o + ty * p.dv + col) = o;
-  __syncthreads();
-  float x = 0.0f;
-  if (tid < p.dv)
-    for (int y = 0; y < ty_n; ++y) x += sh_o[y * p.dv + tid];
-  // GroupNorm over the head's dv outputs, one a thread
-  auto block_sum = [&](float f, int buf) {
-    f = warp_sum(f);
-    if ((tid & 31) == 0) sh_red[buf][tid >> 5] = f;
+  auto ahead = [&](int i, int phase) {            // what the coming phase reads that no phase writes
+    if (phase == 1) {
+      const MixShape m(p);
+      fetch_state(w, p, p.layer[i], m, m.first, m.ty);
+      return;
+    }
+    const Job& j = jobs[i & 1][phase];
+    prefetch<MT>(w, bias, j, share_of(j, tiles[phase]));
+    if (phase == 0 || phase == 3) stage_norm(norm, j);
+  };
+  // Every CTA has arrived (what it wrote is visible), or the wait ran out: the CTA then reports it and leaves.  What the
+  // next phases need besides the others' results is requested between the arrival and the wait.
+  auto arrive = [&]() {
+    ++passed;
     __syncthreads();
-    float s = 0.0f;
-#pragma unroll
-    for (int i = 0; i < WARPS; ++i) s += sh_red[buf][i];
-    return s;
+    if (threadIdx.x == 0) add_release(p.arrived);
   };
-  const float mean = block_sum(x, 0) / (float)p.dv;
-  const float d = tid < p.dv ? x - mean : 0.0f;
-  const float rstd = rsqrtf(block_sum(d * d, 1) / (float)p.dv + p.gn_eps);
-  if (tid < p.dv) p.y[(int64_t)b * width + h * p.dv + tid] = __float2bfloat16_rn(d * rstd * activate(p.act, z));
-}
-
-// Launch with (or, for the first of a chain, without) permission to start before the launch ahead of it has ended.
-template <typename P>
-cudaError_t launch(void (*kernel)(P), dim3 grid, size_t smem, bool chained, const P& p, cudaStream_t stream) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid; cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr; cfg.numAttrs = chained ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, p);
-}
-
-template <int N8, int MT, bool NORM>
-cudaError_t launch_project_t(const ProjectParams& p, int n, bool chained, cudaStream_t stream) {
-  constexpr int RED = WARPS * MT * 16 * (N8 * 8 + 2) * 4;
-  constexpr int MOST = (NORM ? MT * 16 * norm_pitch(MAX_D) : 0) + RED;
-  static_assert(MOST <= 227 * 1024, "shared memory of a CTA");
-  static std::atomic<bool> configured[64];
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
-    const cudaError_t e = cudaFuncSetAttribute(project_kernel<N8, MT, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST);
-    if (e != cudaSuccess) return e;
-    if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
+  auto wait = [&]() {
+    if (threadIdx.x == 0) {
+      const long long t0 = clock64();
+      const unsigned want = passed * gridDim.x;
+      int gone = 0;
+      while (ld_acquire(p.arrived) < want)
+        if (clock64() - t0 > p.wait_cycles) { gone = 1; break; }
+      if (gone) atomicCAS(p.status, 0, 0x7f0);
+      quit = gone;
+    }
+    copy_async_wait();
+    __syncthreads();
+    return quit == 0;
+  };
+  auto grid_meet = [&]() { arrive(); return wait(); };
+  auto grid_sync = [&](int i, int phase) {        // ahead of that phase
+    arrive();
+    ahead(i, phase);
+    request_l2(i, phase + 2);
+    // the records of the layer after: their slot was last read by this layer's predecessor
+    if (phase == 2 && (threadIdx.x >> 5) == WARPS - 1) make_jobs(i + 1);
+    return wait();
+  };
+  ahead(0, 0);
+  request_l2(0, 1);
+  request_l2(0, 2);
+  copy_async_wait();
+  __syncthreads();
+  for (int i = 0; i < p.layers; ++i) {
+    for (int phase = 0; phase < 5; ++phase) {
+      if (phase == 1) {
+        mix(reinterpret_cast<float*>(sm), w, p, p.layer[i]);
+      } else {
+        const Job& j = jobs[i & 1][phase];
+        const Share s = share_of(j, tiles[phase]);
+        if (MT == 1 && (phase == 0 || phase == 3)) {
+          normalise(sm, norm_pitch(j.K), norm, j, threadIdx.x >> 5, WARPS, p.B);
+          __syncthreads();
+          project_any<MT, MT == 1>(sm, w, bias, j, s, p.B);
+        } else {
+          if (MT > 1 && (phase == 0 || phase == 3)) {
+            // warp 0 of the first B CTAs takes a row; everybody reads the result
+            if (threadIdx.x < 32) normalise(reinterpret_cast<uint8_t*>(p.normed), j.K * 2, norm, j, blockIdx.x, gridDim.x, p.B);
+            if (!grid_meet()) return;
+          }
+          project_any<MT, false>(sm, w, bias, j, s, p.B);
+        }
+      }
+      if (i == p.layers - 1 && phase == 4) break;
+      if (!(phase == 4 ? grid_sync(i + 1, 0) : grid_sync(i, phase + 1))) return;
+    }
   }
-  const size_t smem = (NORM ? MT * 16 * norm_pitch(p.K) : 0) + RED;
-  return launch(project_kernel<N8, MT, NORM>, dim3(n / (N8 * 8)), smem, chained, p, stream);
 }
 
-// Rows a CTA owns: as few as still make one CTA an SM or so (128 CTAs for 1024 to 4096 outputs), which spreads a small
-// matrix over the GPU; 32 at most, which is what the registers hold.  Every matrix of the launch is a multiple of them.
-template <int MT, bool NORM>
-cudaError_t launch_project_m(const ProjectParams& p, int n, bool chained, cudaStream_t stream) {
-  auto fits = [&](int nt) {
-    for (int i = 0; i < 4; ++i)
-      if (p.n_end[i] % nt) return false;
-    return true;
-  };
-  if (n > 2 * 8 * 148 && fits(32)) return launch_project_t<4, MT, NORM>(p, n, chained, stream);
-  if (n > 8 * 148 && fits(16)) return launch_project_t<2, MT, NORM>(p, n, chained, stream);
-  return launch_project_t<1, MT, NORM>(p, n, chained, stream);
-}
-template <bool NORM>
-cudaError_t launch_project(const ProjectParams& p, int n, bool chained, cudaStream_t stream) {
-  if (p.B <= 16) return launch_project_m<1, NORM>(p, n, chained, stream);
-  if (p.B <= 32) return launch_project_m<2, NORM>(p, n, chained, stream);
-  return launch_project_m<4, NORM>(p, n, chained, stream);
+template <int MT>
+cudaError_t launch_token(const TokenParams& p, cudaStream_t stream) {
+  constexpr int TPP = MT > 2 ? 2 : 4;
+  constexpr int RED = WARPS * MT * 16 * (TPP * 8 + 2) * 4, MIX = (4 * 512 + THREADS * 4) * 4;
+  constexpr int MOST = NORM_BYTES + (MT == 1 ? 16 * norm_pitch(MAX_D) : 0) + RED;
+  static_assert(MOST <= 227 * 1024 && MIX <= RED, "shared memory of a CTA");
+  static std::atomic<int> sms[64];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  int n = dev >= 0 && dev < 64 ? sms[dev].load(std::memory_order_acquire) : 0;
+  if (n == 0) {
+    if ((e = cudaFuncSetAttribute(token_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64) sms[dev].store(n, std::memory_order_release);
+  }
+  if ((e = cudaMemsetAsync(p.arrived, 0, sizeof(unsigned), stream)) != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(n); cfg.blockDim = dim3(THREADS); cfg.stream = stream;
+  cfg.dynamicSmemBytes = NORM_BYTES + (MT == 1 ? 16 * norm_pitch(p.H * p.dv) : 0) + RED;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeCooperative;        // the CTAs wait for one another: all of them resident, or none starts
+  attr.val.cooperative = 1;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, token_kernel<MT>, p);
 }
 
 bool aligned(const void* p, int n) { return (uintptr_t)p % n == 0; }
@@ -382,7 +604,7 @@ bool aligned(const void* p, int n) { return (uintptr_t)p % n == 0; }
 
 int64_t decoder_token_workspace(const fpb_token_dims& d) {
   const int64_t qk = (int64_t)d.H * d.dk, width = (int64_t)d.H * d.dv;
-  return 2 * (int64_t)d.B * (2 * qk + 2 * width + 3 * width + d.ffn) + 64;     // qkvg | gated | two streams of x | ffn, bf16
+  return 2 * (int64_t)d.B * (2 * qk + 2 * width + 4 * width + d.ffn) + 256;    // TokenParams' buffers, bf16; barrier
 }
 
 int check_decoder_token(const fpb_token_dims& d, const fpb_decoder_layer* layers) {
@@ -403,8 +625,9 @@ int check_decoder_token(const fpb_token_dims& d, const fpb_decoder_layer* layers
     }
     for (const void* b : {l.bq, l.bk, l.bv, l.bg, l.bo, l.b1, l.b2})
       if (!aligned(b, 4)) return FPB_ERR_BAD_STRIDE;
-    for (const float* v : {l.norm1_w, l.norm1_b, l.norm2_w, l.norm2_b, l.phasors})
-      if (!aligned(v, 8)) return FPB_ERR_BAD_STRIDE;
+    for (const float* v : {l.norm1_w, l.norm1_b, l.norm2_w, l.norm2_b})
+      if (!aligned(v, 16)) return FPB_ERR_BAD_STRIDE;
+    if (!aligned(l.phasors, 8)) return FPB_ERR_BAD_STRIDE;
     if (l.act_gate < 0 || l.act_gate > FPB_ACT_RELU || l.act_ffn < 0 || l.act_ffn > FPB_ACT_RELU) return FPB_ERR_BAD_SHAPE;
     if (!l.s_out) return FPB_ERR_NULL_POINTER;
     // rows of four state elements are read and written at a time
@@ -418,64 +641,36 @@ int check_decoder_token(const fpb_token_dims& d, const fpb_decoder_layer* layers
 
 int launch_decoder_token(const fpb_token_dims& d, const fpb_decoder_layer* layers, const float* gamma, const void* x, int64_t x_stride,
                          void* y, int64_t y_stride, cudaStream_t stream, int* n_launched) {
-  const int width = d.H * d.dv, qk = d.H * d.dk, n4 = 2 * qk + 2 * width;
+  const int width = d.H * d.dv, qk = d.H * d.dk;
+  TokenParams p;
+  p.B = d.B; p.H = d.H; p.dk = d.dk; p.dv = d.dv; p.ffn = d.ffn;
+  p.prev_f32 = d.prev_dtype == FPB_F32; p.out_f32 = d.out_dtype == FPB_F32;
   bf16* buf = (bf16*)d.workspace;
-  auto take = [&](int64_t n) { bf16* r = buf; buf += (n + 7) / 8 * 8; return r; };
-  bf16* qkvg = take((int64_t)d.B * n4);
-  bf16* gated = take((int64_t)d.B * width);
-  bf16* mid = take((int64_t)d.B * width);         // x + retention of the layer
-  bf16* stream_x = take((int64_t)d.B * width);    // x between layers
-  bf16* hidden = take((int64_t)d.B * d.ffn);
-  const bf16* in = (const bf16*)x; int64_t in_stride = x_stride;
-  bool chained = false;
-  cudaError_t e = cudaSuccess;
-  for (int i = 0; i < d.layers && e == cudaSuccess; ++i) {
-    const fpb_decoder_layer& l = layers[i];
-    ProjectParams p{};
-    p.B = d.B; p.K = width; p.act = FPB_ACT_NONE;
-    p.x = in; p.x_stride = in_stride; p.norm_w = l.norm1_w; p.norm_b = l.norm1_b; p.eps = (float)l.norm1_eps;
-    p.w[0] = (const bf16*)l.wq; p.w[1] = (const bf16*)l.wk; p.w[2] = (const bf16*)l.wv; p.w[3] = (const bf16*)l.wg;
-    p.bias[0] = (const bf16*)l.bq; p.bias[1] = (const bf16*)l.bk; p.bias[2] = (const bf16*)l.bv; p.bias[3] = (const bf16*)l.bg;
-    p.n_end[0] = qk; p.n_end[1] = 2 * qk; p.n_end[2] = 2 * qk + width; p.n_end[3] = n4;
-    p.y = qkvg; p.y_stride = n4;
-    if ((e = launch_project<true>(p, n4, chained, stream)) != cudaSuccess) break;
-    chained = true;
-
-    MixParams mx;
-    mx.qkvg = qkvg; mx.phasors = (const float2*)l.phasors;
-    mx.s_prev = l.s_prev; mx.prev_sb = l.prev_sb; mx.prev_sh = l.prev_sh;
-    mx.s_out = l.s_out; mx.out_sb = l.out_sb; mx.out_sh = l.out_sh;
-    mx.y = gated; mx.H = d.H; mx.dk = d.dk; mx.dv = d.dv; mx.act = (int)l.act_gate; mx.gn_eps = (float)l.gn_eps;
-    for (int h = 0; h < d.H; ++h) mx.gamma[h] = gamma[h];
-    const dim3 mgrid(d.H, d.B);
-    if (d.out_dtype == FPB_F32)
-      e = d.prev_dtype == FPB_F32 ? launch(mix_kernel<float, float>, mgrid, 0, true, mx, stream) : launch(mix_kernel<bf16, float>, mgrid, 0, true, mx, stream);
-    else
-      e = d.prev_dtype == FPB_F32 ? launch(mix_kernel<float, bf16>, mgrid, 0, true, mx, stream) : launch(mix_kernel<bf16, bf16>, mgrid, 0, true, mx, stream);
-    if (e != cudaSuccess) break;
-
-    auto one = [&](const bf16* src, int K, const void* w, const void* b, int n) {      // a launch of one matrix
-      ProjectParams r{};
-      r.B = d.B; r.K = K; r.act = FPB_ACT_NONE; r.x = src; r.x_stride = K;
-      r.w[0] = (const bf16*)w; r.bias[0] = (const bf16*)b;
-      for (int j = 0; j < 4; ++j) r.n_end[j] = n;
-      return r;
-    };
-    ProjectParams po = one(gated, width, l.wo, l.bo, width);
-    po.residual = in; po.res_stride = in_stride; po.y = mid; po.y_stride = width;
-    if ((e = launch_project<false>(po, width, true, stream)) != cudaSuccess) break;
-    ProjectParams p1 = one(mid, width, l.w1, l.b1, d.ffn);
-    p1.norm_w = l.norm2_w; p1.norm_b = l.norm2_b; p1.eps = (float)l.norm2_eps; p1.act = (int)l.act_ffn;
-    p1.y = hidden; p1.y_stride = d.ffn;
-    if ((e = launch_project<true>(p1, d.ffn, true, stream)) != cudaSuccess) break;
-    ProjectParams p2 = one(hidden, d.ffn, l.w2, l.b2, width);
-    const bool last = i == d.layers - 1;
-    p2.residual = mid; p2.res_stride = width; p2.y = last ? (bf16*)y : stream_x; p2.y_stride = last ? y_stride : width;
-    e = launch_project<false>(p2, width, true, stream);
-    in = stream_x; in_stride = width;
-    *n_launched += 5;
+  p.arrived = (unsigned*)buf; buf += 64;
+  auto take = [&](int64_t n) { bf16* r = buf; buf += n; return r; };       // (every row is a multiple of 16 bytes)
+  p.qkvg = take((int64_t)d.B * (2 * qk + 2 * width));
+  p.gated = take((int64_t)d.B * width);
+  p.mid = take((int64_t)d.B * width);             // x + retention of the layer
+  p.between = take((int64_t)d.B * width);         // x between layers
+  p.hidden = take((int64_t)d.B * d.ffn);
+  p.normed = take((int64_t)d.B * width);
+  p.status = device_status_ptr();
+  p.wait_cycles = walk_tuning().wait_cycles;
+  if (!p.status) return FPB_ERR_LAUNCH;
+  for (int h = 0; h < d.H; ++h) p.gamma[h] = gamma[h];
+  for (int i0 = 0; i0 < d.layers; i0 += MAX_LAYERS) {
+    const bool last = i0 + MAX_LAYERS >= d.layers;
+    p.layers = last ? d.layers - i0 : MAX_LAYERS;
+    // a launch after the first starts from the stream of x that the one before it ended in (`between` is next written by
+    // the last phase of its first layer, long after everyone has read it)
+    p.x = i0 == 0 ? (const bf16*)x : p.between; p.x_stride = i0 == 0 ? x_stride : width;
+    p.y = last ? (bf16*)y : p.between; p.y_stride = last ? y_stride : width;
+    for (int i = 0; i < p.layers; ++i) p.layer[i] = layers[i0 + i];
+    const cudaError_t e = d.B <= 16 ? launch_token<1>(p, stream) : d.B <= 32 ? launch_token<2>(p, stream) : launch_token<4>(p, stream);
+    if (e != cudaSuccess) return FPB_ERR_LAUNCH;
+    ++*n_launched;
   }
-  return e == cudaSuccess ? FPB_OK : FPB_ERR_LAUNCH;
+  return FPB_OK;
 }
 
 }  // namespace fpb

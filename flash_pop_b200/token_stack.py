@@ -1,4 +1,4 @@
-"""One token through a stack of pre-norm decoder layers as a chain of fused launches (``fpb_decoder_token``): what
+"""One token through a stack of pre-norm decoder layers in one cooperative launch (``fpb_decoder_token``): what
 ``RetNetDecoder.forward_recurrent`` (flash_pop/retnet.py:535-546) runs when every layer is the plain one and nothing is
 watching - no gradient, no hook on a sub-module, no replaced sub-module, no autocast or dispatch mode, bf16 weights and
 activations, at most 64 rows.  Everything else takes the layer-by-layer path.  Nothing is remembered between calls: the
@@ -119,7 +119,7 @@ def _layer(layer, first, shape, x_device, index, layer_cls, retention_cls):
 
 
 def decoder_token(net, x: Tensor, recurrent_state: Optional[RecurrentState], layer_cls, retention_cls):
-    """``net.forward_recurrent(x, recurrent_state)`` through the fused launches, or None when the call is not one of theirs."""
+    """``net.forward_recurrent(x, recurrent_state)`` through the fused launch, or None when the call is not one of theirs."""
     if _watched() or type(x) is not Tensor or not x.is_cuda or x.dtype != _BF or x.dim() != 2 or not x.is_contiguous():
         return None
     B, device = x.shape[0], x.device

@@ -230,7 +230,8 @@ int64_t fpb_decoder_token_workspace(const fpb_token_dims* dims);
  * flash_pop/retnet.py:535-546; RetNetDecoderLayer.forward_recurrent and MultiScaleRetention.forward_recurrent below it):
  *   x <- x + out_proj(GroupNorm(retention step(rotate(q), rotate(k), v)) . act(gate)),   x <- x + linear2(act(linear1(norm(x))))
  * x, y: (B, H dv) bf16 rows, row pitches in elements.  At most 64 rows, H dv <= 1024 and a multiple of 32, ffn a multiple
- * of 32, H dk of 8, dv of 4, dk even; FPB_ERR_BAD_SHAPE outside.  Five launches per layer, no allocation, no synchronisation.
+ * of 32, H dk of 8, dv of 4, dk even; FPB_ERR_BAD_SHAPE outside.  One cooperative launch per 16 layers, no allocation, no
+ * synchronisation with the host.
  */
 int fpb_decoder_token(const fpb_token_dims* dims, const fpb_decoder_layer* layers, const void* x, int64_t x_stride,
                       void* y, int64_t y_stride, fpb_stream_t stream);
