@@ -464,25 +464,23 @@ __global__ void __launch_bounds__(BCfg<DK, DV>::NTHREADS, 1) bwd_fused_kernel(co
     constexpr std::true_type scratch_t{};
     constexpr int esz = SF32 ? 4 : 2;
     auto at = [&](const void* base, int64_t elems) { return (void*)((const char*)base + elems * esz); };
-    // suffix calls: the batch index is (row, group of sfx_G consecutive suffixes); the walk goes through the group's
-    // suffixes from the last to the first, and what it carries when it leaves suffix m is the gradient of the state
-    // that suffix started from
+    // suffix calls: suffix f of the call is suffix f % M of row f / M; the walk goes through its piece's suffixes from the
+    // last to the first, and what it carries when it leaves one is the gradient of the state that suffix started from
     // (Grouping is compiled into the 64 x 64 kernel only - the shape suffixes come in; in the larger tiles its few
     // extra live registers spill the state, which costs the long-sequence workloads far more than grouping gains.)
     constexpr bool GROUPED = DK == 64 && DV == 64;
     const int sfx_g = GROUPED ? p.sfx_G : 1;
-    const int groups = p.sfx_M > 0 ? p.sfx_M / sfx_g : 1;
-    auto sfx_grad = [&](int m) -> void* {
-      const int sfx_row = b / groups;
-      if (m == 0) return p.g_end ? at(p.g_end, sfx_row * p.ge_sb + h * p.ge_sh) : nullptr;
-      return p.sfx_blocks ? at(p.sfx_blocks, (((int64_t)sfx_row * p.sfx_N + (m - 1)) * p.H + h) * state_elems) : nullptr;
+    auto sfx_grad = [&](int f) -> void* {
+      const int row = f / p.sfx_M, m = f % p.sfx_M;
+      if (m == 0) return p.g_end ? at(p.g_end, row * p.ge_sb + h * p.ge_sh) : nullptr;
+      return p.sfx_blocks ? at(p.sfx_blocks, (((int64_t)row * p.sfx_N + (m - 1)) * p.H + h) * state_elems) : nullptr;
     };
-    if (p.n_seg > 1) {
+    if (p.n_seg > 1 && p.sfx_M == 0) {
       // T-segments: G after this piece's last token was put into fp32 scratch by the scan; the first piece ends in dS_0
       x_start = p.seg_states + (((int64_t)b * p.H + h) * p.n_seg + seg) * state_elems;
       if (seg == 0 && p.g_end) x_end = at(p.g_end, b * p.ge_sb + h * p.ge_sh);
     } else if (p.sfx_M > 0) {
-      if (sfx_g == 1) x_end = sfx_grad(b % groups);    // grouped walks store at every suffix start, inside the loop
+      if (sfx_g == 1) x_end = sfx_grad(b);             // grouped walks store at every suffix start, inside the loop
     } else {
       if (p.g_start) x_start = at(p.g_start, b * p.gs_sb + h * p.gs_sh);
       if (p.g_end) x_end = at(p.g_end, b * p.ge_sb + h * p.ge_sh);
@@ -655,7 +653,7 @@ __global__ void __launch_bounds__(BCfg<DK, DV>::NTHREADS, 1) bwd_fused_kernel(co
     };
 
     if (x_start) {
-      if (p.n_seg > 1) load_global(x_start, scratch_t, false);
+      if (p.n_seg > 1 && p.sfx_M == 0) load_global(x_start, scratch_t, false);
       else load_global(x_start, state_t, false);
     }
     else {
@@ -700,7 +698,7 @@ __global__ void __launch_bounds__(BCfg<DK, DV>::NTHREADS, 1) bwd_fused_kernel(co
           mbar_arrive(bar(B_DSFREE + (n_u & 1)));
           ++n_u;
           if (GROUPED && sfx_g > 1 && ck_u.a % p.block_size == 0) {   // that was the first chunk of a suffix
-            void* dst = sfx_grad((b % groups) * sfx_g + ck_u.a / p.block_size);
+            void* dst = sfx_grad(ck_u.a / p.block_size);
             if (dst) store_global(dst);
 #pragma unroll
             for (int i = 0; i < G::NS; ++i) S[i] = 0.f;      // the suffix before it ends in a state nobody reads
@@ -772,26 +770,26 @@ int launch_bwd_fused(const UmmaBwdArgs& a, cudaStream_t stream, int* n_launched)
   int r;
   int B = a.B, T = a.T, block_size = a.block_size;
   const int H = a.H;
-  // suffix calls: G consecutive suffixes of a row as one sequence per CTA (see launch_one in retention_scan_sm100.cu)
+  // suffix calls: all suffixes of a head as one sequence in pieces of G (see launch_one in retention_scan_sm100.cu)
   SeqView q = a.q, k = a.k, v = a.v, dO = a.dO, dK = a.dK, dV = a.dV;
   int G = 1;
-  if (a.sfx_grad.M > 1 && a.block_size == 0) {
-    bool contiguous = true;
-    for (const SeqView* s : {&q, &k, &v, &dO, &dK, &dV}) contiguous = contiguous && s->sb == (int64_t)T * s->st;
-    if (contiguous && a.dk == 64 && a.dv == 64) G = choose_suffix_group(a.sfx_grad.M, (long long)(B / a.sfx_grad.M) * H);
+  Segments sg{1, 0};
+  if (a.sfx_grad.M > 0 && a.block_size == 0 && a.dk == 64 && a.dv == 64 && (int64_t)B * T <= (1 << 30)) {
+    bool joined = true;
+    for (const SeqView* s : {&q, &k, &v, &dO, &dK, &dV}) joined = joined && (B == 1 || s->sb == (int64_t)T * s->st);
+    if (joined) G = choose_suffix_group(B, H, 1);
     if (G > 1) {
-      B /= G; block_size = T; T *= G;
-      for (SeqView* s : {&q, &k, &v, &dO, &dK, &dV}) s->sb *= G;
+      sg = Segments{(B + G - 1) / G, G * T};
+      block_size = T; T *= B; B = 1;
     }
   }
   // under-filled: cut the sequences into T-segments (segment_scan.cu) - local values of G per piece from a reverse
   // state-only walk over (Q, dO), the scan (which also writes dS_0), then this kernel once per piece
-  Segments sg{1, 0};
   if (segments_enabled() && a.scratch && a.sfx_grad.M == 0) {
     const int align = a.block_size > 0 ? C / gcd_int(C, a.block_size) * a.block_size : C;
     sg = choose_segments((long long)H * B * (dv_halves ? 2 : 1), 1, T, align, (long long)B * H, (long long)a.dk * a.dv, a.scratch_bytes, B);
   }
-  if (sg.n > 1) {
+  if (sg.n > 1 && a.sfx_grad.M == 0) {
     if ((r = launch_segment_states(a.q, a.dO, true, a.d_block_states, a.gamma, B, T, H, a.dk, a.dv, a.block_size, a.n_blocks,
                                    a.state_f32, sg, a.scratch, stream)) != FPB_OK)
       return r;
@@ -812,7 +810,7 @@ int launch_bwd_fused(const UmmaBwdArgs& a, cudaStream_t stream, int* n_launched)
   }
   p.dk_out = (bf16*)dK.data; p.dk_sb = dK.sb; p.dk_st = dK.st; p.dk_sh = dK.sh;
   p.dv_out = (bf16*)dV.data; p.dv_sb = dV.sb; p.dv_st = dV.st; p.dv_sh = dV.sh;
-  const bool split = sg.n > 1;
+  const bool split = sg.n > 1 && a.sfx_grad.M == 0;
   p.g_start = split ? nullptr : a.d_s_out.data; p.gs_sb = a.d_s_out.sb; p.gs_sh = a.d_s_out.sh;
   p.g_end = a.d_s0.data; p.ge_sb = a.d_s0.sb; p.ge_sh = a.d_s0.sh;      // split: written by the piece the walk reaches last
   p.block_grads = a.d_block_states;

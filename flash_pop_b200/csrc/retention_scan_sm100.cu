@@ -50,8 +50,9 @@
 // proper then runs one CTA per (batch, head, tile, segment) from its start state in fp32 scratch memory.
 //
 // Suffix calls (thousands of sequences of a few chunks, each starting from its own state and dropping its end
-// state) may be regrouped by the launcher: G consecutive suffixes of a row as one sequence of G*T tokens with block
-// size T, the state replaced at every suffix start - same results, one CTA set-up per G suffixes.
+// state) may be regrouped by the launcher: where all suffixes of the call follow one another in memory they are ONE
+// sequence per head, cut into pieces of G suffixes (block size = suffix length, the state replaced at every suffix
+// start) - same results, and as many CTAs as fit the GPU at once, each with its even share.
 //
 // dv = 256 beside dk = 128.  A MODE_DQ walk may cut dv instead of dk (ScanParams::col_split): two CTAs per head on the
 // 128 x 128 instance, each with its half of the state columns; its output tile is then a partial sum, which the TMA
@@ -778,14 +779,13 @@ FPB_UNROLL_MMA
     constexpr std::true_type scratch_t{};
     constexpr int esz = SF32 ? 4 : 2;
     auto at = [&](const void* base, int64_t elems) { return (void*)((const char*)base + elems * esz); };
-    // suffix calls: the batch index is (row, group of sfx_G consecutive suffixes)
-    const int groups = p.sfx_M > 0 ? p.sfx_M / p.sfx_G : 1;
-    const int sfx_row = b / groups, sfx_m0 = (b % groups) * p.sfx_G;
-    auto sfx_start = [&](int m) -> const void* {       // where suffix m of this row starts from (forward walks)
-      if (m == 0) return p.s0 ? at(p.s0, sfx_row * p.s0_sb + h * p.s0_sh) : nullptr;
-      return p.sfx_blocks ? at(p.sfx_blocks, (((int64_t)sfx_row * p.sfx_N + (m - 1)) * p.H + h) * state_elems) : nullptr;
+    // suffix calls: suffix f of the call is suffix f % M of row f / M; grouped, the piece's first one is t0 / block_size
+    auto sfx_start = [&](int f) -> const void* {       // where suffix f starts from (forward walks)
+      const int row = f / p.sfx_M, m = f % p.sfx_M;
+      if (m == 0) return p.s0 ? at(p.s0, row * p.s0_sb + h * p.s0_sh) : nullptr;
+      return p.sfx_blocks ? at(p.sfx_blocks, (((int64_t)row * p.sfx_N + (m - 1)) * p.H + h) * state_elems) : nullptr;
     };
-    if (SO || p.n_seg > 1) {
+    if (SO || (p.n_seg > 1 && p.sfx_M == 0)) {
       // T-segments: a STATE_ONLY pass leaves the local end value in this segment's scratch slot; the walk proper
       // starts from the value the scan put there, and the piece it reaches last ends in the call's end state
       float* slot = p.seg_states + (((int64_t)b * p.H + h) * p.n_seg + seg) * state_elems;
@@ -795,9 +795,9 @@ FPB_UNROLL_MMA
         if (seg == (REV ? 0 : p.n_seg - 1) && p.s_out) x_end = at(p.s_out, b * p.so_sb + h * p.so_sh);
       }
     } else if (p.sfx_M > 0) {
-      const int row = sfx_row, m = sfx_m0;
+      const int f = p.sfx_G > 1 ? t0 / p.block_size : b, row = f / p.sfx_M, m = f % p.sfx_M;
       void* blk = (m > 0 && p.sfx_blocks) ? at(p.sfx_blocks, (((int64_t)row * p.sfx_N + (m - 1)) * p.H + h) * state_elems) : nullptr;
-      if (!REV) x_start = sfx_start(m);
+      if (!REV) x_start = sfx_start(f);
       else x_end = m == 0 ? (p.s_out ? at(p.s_out, row * p.so_sb + h * p.so_sh) : nullptr) : blk;
     } else {
       if (p.s0) x_start = at(p.s0, b * p.s0_sb + h * p.s0_sh);
@@ -937,7 +937,7 @@ FPB_UNROLL_MMA
     };
 
     if (x_start) {
-      if (!SO && p.n_seg > 1) load_global(x_start, scratch_t, false);
+      if (!SO && p.n_seg > 1 && p.sfx_M == 0) load_global(x_start, scratch_t, false);
       else load_global(x_start, state_t, false);
     }
     else {
@@ -1035,7 +1035,7 @@ FPB_UNROLL_MMA
           advance<REV>(ck_u, t_end, p.sched_bs);
           if (!REV && !SO && p.sfx_G > 1 && ck_u.a % p.block_size == 0) {
             // grouped suffixes: the next chunk opens the next suffix, which starts from its own state
-            const void* src = sfx_start(sfx_m0 + ck_u.a / p.block_size);
+            const void* src = sfx_start(ck_u.a / p.block_size);
             if (src) load_global(src, state_t, false);
             else {
 #pragma unroll
@@ -1158,8 +1158,8 @@ int launch_scan(const ScanParams& p, bool rev, bool state_only, dim3 grid, cudaS
 #define FPB_KNOB constexpr int
 #endif
 FPB_KNOB g_tile_pref = 1;            // 1: 128x128 state tiles where they apply; 0: 64-wide tiles (two CTAs per SM)
-FPB_KNOB g_sfx_group = 16;           // most suffixes one CTA walks back to back (1: one CTA per suffix)
-FPB_KNOB g_sfx_min_ctas = 3 * 296;   // ... as long as that many CTAs remain (three waves of two CTAs per SM)
+FPB_KNOB g_sfx_group = 1 << 20;      // most suffixes one CTA walks back to back (1: one CTA per suffix)
+FPB_KNOB g_sfx_slots = 0;            // CTAs they are shared out over (0: what fits the GPU at once)
 FPB_KNOB g_pop_emit = 1;             // 1: POP forward walks over full chunks where block states can come from partial increments
 FPB_KNOB g_fused_bwd = 1;            // 1: dK, dV, dS_0 in one fused reverse walk where it applies; 0: two separate walks
 FPB_KNOB g_segments = 1;             // 1: under-filled launches are cut into T-segments when the caller gave scratch memory
@@ -1238,6 +1238,8 @@ __global__ void __launch_bounds__(256) zero_seq_kernel(bf16* base, int64_t sb, i
   }
 }
 
+constexpr int64_t kMaxJoinedTokens = 1 << 30;   // token positions are 32-bit
+
 int gcd_int(int a, int b) { while (b) { const int t = a % b; a = b; b = t; } return a; }
 
 // One launch of the kernel: the walk itself, or (state_only) the local end values of its T-segments.
@@ -1247,19 +1249,19 @@ int launch_one(const PassArgs& a, Segments sg, bool state_only, cudaStream_t str
   const int B = a.B, T = a.T, H = a.H, dk = a.dk, dv = a.dv;
   ScanParams p;
   int r;
-  // Suffix calls are thousands of sequences of a few chunks.  Where the suffixes of a row follow one another in
-  // memory, G of them are walked by one CTA as one sequence of G * T tokens whose state is replaced at every suffix
-  // start (block size = suffix length, so no chunk straddles two suffixes): the CTA's set-up and pipeline fill are
-  // paid once per G suffixes.  G is the largest divisor of M that still leaves a few waves of CTAs.
+  const Tiling t = tiling_of(mode, dk, dv, col_split_ok(mode, a.block_size, a.sfx));
+  // Suffix calls are thousands of sequences of a few chunks.  Where all of them follow one another in memory they are
+  // walked as one sequence per head and tile, in pieces of G suffixes whose state is replaced at every suffix start (block
+  // size = suffix length, so no chunk straddles two suffixes): the CTA's set-up and pipeline fill are paid once per G.
   int G = 1;
   SeqView x = state_only ? a.k : a.x, k = a.k, v = a.v, out = state_only ? a.v : a.out;   // a state-only pass reads k and v only
   int Bk = B, Tk = T, block_size = a.block_size;
-  if (a.sfx.M > 1 && !a.rev && g_sfx_group && a.block_size == 0 && x.sb == (int64_t)T * x.st && k.sb == (int64_t)T * k.st &&
-      v.sb == (int64_t)T * v.st && out.sb == (int64_t)T * out.st) {
-    G = choose_suffix_group(a.sfx.M, (long long)(B / a.sfx.M) * H * (mode == MODE_FWD ? (dv + 127) / 128 : (dk + 127) / 128));
+  auto joined = [&](const SeqView& s) { return B == 1 || s.sb == (int64_t)T * s.st; };
+  if (a.sfx.M > 0 && !a.rev && a.block_size == 0 && (int64_t)B * T <= kMaxJoinedTokens && joined(x) && joined(k) && joined(v) && joined(out)) {
+    G = choose_suffix_group(B, (long long)H * t.tiles, t.ctas_per_sm);
     if (G > 1) {
-      Bk = B / G; Tk = T * G; block_size = T;
-      x.sb *= G; k.sb *= G; v.sb *= G; out.sb *= G;
+      sg = Segments{(B + G - 1) / G, G * T};
+      Bk = 1; Tk = B * T; block_size = T;
     }
   }
   if ((r = make_seq_map(&p.map_x, x, Bk, Tk, H, xw, C)) != FPB_OK) return r;
@@ -1267,7 +1269,7 @@ int launch_one(const PassArgs& a, Segments sg, bool state_only, cudaStream_t str
   if ((r = make_seq_map(&p.map_v, v, Bk, Tk, H, dv, C)) != FPB_OK) return r;
   if ((r = make_seq_map(&p.map_out, out, Bk, Tk, H, ow, 16)) != FPB_OK) return r;   // one score warp's 16 rows
   p.out = (bf16*)out.data; p.out_sb = out.sb; p.out_st = out.st; p.out_sh = out.sh;
-  const bool split = sg.n > 1;
+  const bool split = sg.n > 1 && a.sfx.M == 0;
   // a segmented walk starts from the scratch slots; its last piece writes the end value
   p.s0 = split ? nullptr : a.start.data; p.s0_sb = a.start.sb; p.s0_sh = a.start.sh;
   p.s_out = state_only ? nullptr : a.end.data; p.so_sb = a.end.sb; p.so_sh = a.end.sh;
@@ -1288,7 +1290,6 @@ int launch_one(const PassArgs& a, Segments sg, bool state_only, cudaStream_t str
   if (!p.status) return FPB_ERR_LAUNCH;
   for (int h = 0; h < H; ++h) p.log2g[h] = (float)std::log2((double)a.gamma[h]);
 
-  const Tiling t = tiling_of(mode, dk, dv, col_split_ok(mode, a.block_size, a.sfx));
   p.col_split = t.col_split ? 1 : 0;
   const dim3 grid(t.tiles, H, Bk * (state_only ? sg.n - 1 : sg.n));
 #define FPB_SCAN_CASE(MODE_, R_, CC_) \
@@ -1337,10 +1338,17 @@ void launch_zero_seq(const SeqView& v, int B, int T, int H, int d, cudaStream_t 
 }
 
 
-int choose_suffix_group(int M, long long units) {
-  for (int cand = g_sfx_group; cand > 1; --cand)
-    if (M % cand == 0 && units * (M / cand) >= g_sfx_min_ctas) return cand;
-  return 1;
+// The CTAs that fit the GPU at once, dealt out over the heads and tiles, share the suffixes evenly.  (Before, a CTA took a
+// divisor of M, at most 16, that left three waves: 1024 suffixes of 80 tokens per head, 8 heads, d = 64 were 8 a CTA in 3.46
+// waves, i.e. 32 suffixes a slot instead of 28 and four set-ups instead of one: forward 180 -> 156 us, dQ 166 -> 147.)
+// One each where that fits: no grouping.
+int choose_suffix_group(int suffixes, long long units, int ctas_per_sm) {
+  if (g_sfx_group <= 1) return 1;
+  const long long slots = g_sfx_slots > 0 ? g_sfx_slots : (long long)sm_count_cached() * ctas_per_sm;
+  long long n = slots / units;
+  if (n < 1) n = 1;
+  const long long G = (suffixes + n - 1) / n;
+  return (int)(G < g_sfx_group ? G : g_sfx_group);
 }
 
 #ifdef FPB_DIAGNOSTICS
@@ -1349,8 +1357,9 @@ int choose_suffix_group(int M, long long units) {
 extern "C" void fpb_debug_trace(void* device_buffer) { g_trace = (long long*)device_buffer; }
 // Choose between the 128x128 state tiles (1, default) and the 64-wide ones (0).
 extern "C" void fpb_debug_tile_pref(int wide) { g_tile_pref = wide; }
-// Upper limit of the suffixes one CTA walks back to back (1 = one CTA per suffix) and the number of CTAs that must remain.
-extern "C" void fpb_debug_suffix_group(int g, int min_ctas) { g_sfx_group = g < 1 ? 1 : g; if (min_ctas > 0) g_sfx_min_ctas = min_ctas; }
+// Upper limit of the suffixes one CTA walks back to back (1 = one CTA per suffix) and the number of CTAs they are shared out
+// over (0: what fits the GPU at once).
+extern "C" void fpb_debug_suffix_group(int g, int slots) { g_sfx_group = g < 1 ? 1 : g; g_sfx_slots = slots; }
 // 0 makes every POP forward walk cut its chunks at block ends.
 extern "C" void fpb_debug_pop_emit(int on) { g_pop_emit = on; }
 // 0 runs the dV and dK walks as two launches instead of the fused reverse kernel.

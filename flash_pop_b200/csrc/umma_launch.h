@@ -45,9 +45,8 @@ bool segments_enabled();
 bool col_split_enabled();
 // zeros over the (B, T, H, d) bf16 elements of a strided view (d a multiple of 8, 16-byte aligned rows)
 void launch_zero_seq(const SeqView& v, int B, int T, int H, int d, cudaStream_t stream);
-// How many consecutive suffixes of a row one CTA walks as one sequence: the largest divisor of M (up to a limit)
-// that leaves enough CTAs to fill the GPU a few times over; `units` = CTAs per suffix index (rows x heads x tiles).
-int choose_suffix_group(int M, long long units);
+// How many consecutive suffixes one CTA walks as one sequence; `units` = heads x tiles, each with all `suffixes`.
+int choose_suffix_group(int suffixes, long long units, int ctas_per_sm);
 // diagnostics: device buffer for per-chunk time stamps, or null
 long long* debug_trace_ptr();
 
