@@ -383,15 +383,8 @@ __global__ void __launch_bounds__(THREADS) chunk_bwd_kernel(const __grid_constan
   if (rev && seg == 0 && p.g_out.data) store_state<DK, DV>(S, (float*)p.g_out.data + b * p.g_out.sb + h * p.g_out.sh, p.dk, p.dv);
 }
 
-template <typename K>
-cudaError_t launch(K kernel, dim3 grid, size_t smem, bool chained, const ChunkParams& p, cudaStream_t stream) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid; cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr; cfg.numAttrs = chained ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, p);
+cudaError_t launch(void (*kernel)(ChunkParams), dim3 grid, size_t smem, bool chained, const ChunkParams& p, cudaStream_t stream) {
+  return launch_kernel(kernel, grid, THREADS, smem, chained, p, stream);
 }
 
 enum Pass { SEGMENTS, FORWARD, BACKWARD };

@@ -127,6 +127,19 @@ Segments choose_segments(long long units, int ctas_per_sm, int T, int align, lon
 int launch_segment_combine(float* seg, Segments sg, int B, int T, int H, int dk, int dv, const float* gamma, bool reverse,
                            StateView start, bool state_f32, cudaStream_t stream);
 
+// Launch `kernel`; `chained`: it may start before the launch ahead of it has ended (programmatic dependent launch) and
+// waits inside, with griddepcontrol.wait, where it needs that launch's results.
+template <typename P>
+cudaError_t launch_kernel(void (*kernel)(P), dim3 grid, int threads, size_t smem, bool chained, const P& p, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr; cfg.numAttrs = chained ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, p);
+}
+
 // Device status word shared by all kernels: 0 = fine; otherwise (role << 8 | barrier id) of the
 // first bounded wait that gave up.
 int32_t* device_status_ptr();

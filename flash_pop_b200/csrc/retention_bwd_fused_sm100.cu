@@ -652,6 +652,7 @@ __global__ void __launch_bounds__(BCfg<DK, DV>::NTHREADS, 1) bwd_fused_kernel(co
       mbar_arrive(bar(B_VRDY + s));
     };
 
+    if (p.n_seg > 1 && p.sfx_M == 0) grid_dep_wait();    // T-segments: the scan may still be running
     if (x_start) {
       if (p.n_seg > 1 && p.sfx_M == 0) load_global(x_start, scratch_t, false);
       else load_global(x_start, state_t, false);
@@ -740,8 +741,8 @@ int launch_fused_t(const BwdParams& p, dim3 grid, cudaStream_t stream) {
       return FPB_ERR_LAUNCH;
     if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
   }
-  bwd_fused_kernel<DK, DV, SF32><<<grid, G::NTHREADS, G::SMEM, stream>>>(p);
-  return FPB_OK;
+  const bool chained = p.n_seg > 1 && p.sfx_M == 0;             // behind the scan over its segments
+  return launch_kernel(bwd_fused_kernel<DK, DV, SF32>, grid, G::NTHREADS, G::SMEM, chained, p, stream) == cudaSuccess ? FPB_OK : FPB_ERR_LAUNCH;
 }
 
 bool state_ok(const StateView& s, bool f32) {

@@ -204,6 +204,7 @@ scan_kernel(const __grid_constant__ ScanParams p) {
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + G::OFF_BAR + OFF_ABORT);
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + G::OFF_BAR + OFF_TMEM_SLOT);
 
+  if (SO) grid_dep_release();                          // the scan over the segments may be set up
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int tile = blockIdx.x, h = blockIdx.y;
   // (a STATE_ONLY pass covers all pieces but the one the walk reaches last - the last one forward, the first one in
@@ -936,6 +937,8 @@ FPB_UNROLL_MMA
       warp_arrive(bar(B_VRDY + s));
     };
 
+    // T-segments: the scan may still be running, and everything up to here - tiles, scores - goes on beside it
+    if (!SO && p.n_seg > 1 && p.sfx_M == 0) grid_dep_wait();
     if (x_start) {
       if (!SO && p.n_seg > 1 && p.sfx_M == 0) load_global(x_start, scratch_t, false);
       else load_global(x_start, state_t, false);
@@ -1111,8 +1114,8 @@ int launch_scan_t(const ScanParams& p, dim3 grid, cudaStream_t stream) {
       return FPB_ERR_LAUNCH;
     if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
   }
-  scan_kernel<MODE, REV, R, CC, SO, SF32, DEEP><<<grid, G::NTHREADS, G::SMEM, stream>>>(p);
-  return FPB_OK;
+  const bool chained = !SO && p.n_seg > 1 && p.sfx_M == 0;      // behind the scan over its segments
+  return launch_kernel(scan_kernel<MODE, REV, R, CC, SO, SF32, DEEP>, grid, G::NTHREADS, G::SMEM, chained, p, stream) == cudaSuccess ? FPB_OK : FPB_ERR_LAUNCH;
 }
 int sm_count_cached() {
   static std::atomic<int> cache[64];
