@@ -10,8 +10,8 @@
 //   dK        dK_j = rs sum_{i>=j} gamma^(i-j) (dO_i . v_j) q_i + gamma^(L-1-j) rs G v_j
 // and T-segments of whole chunks fill the GPU: a pass over the segments' local end values, a scan over them, the walk
 // proper with one CTA per (segment, head, row), dQ and dK/dV side by side in the backward.  The three launches are
-// chained by programmatic dependent launch.  Sums run over 32 tokens and then over chunks, shorter chains than a token at
-// a time: the distance from 64 bits falls (2.3e-7 to 3.2e-7 -> 2.1e-7 at T = 256).
+// chained by programmatic dependent launch.  Every sum is made in runs of at most 32 products that are added up afterwards
+// (as one chain of 128 the distance from 64 bits grew with the head dimension, 1.9e-7 -> 2.4e-7 at 128).
 // Measured, token walk -> chunks, forward | backward: B=2 H=4 T=256 d=64 119 -> 14.5 | 354 -> 24.7 us; B=4 H=8 T=1024
 // d=128 742 -> 193 | 2733 -> 450; B=64 H=16 T=256 d=64 552 -> 302 | 1657 -> 832.
 //
@@ -84,7 +84,7 @@ template <int DK, int DV> __device__ __forceinline__ void update_state(float* S,
 #pragma unroll
   for (int r = 0; r < TR; ++r)
 #pragma unroll
-    for (int c = 0; c < TC; ++c) acc[r][c] = decay * s0[r * (DV + 4) + (c / CV) * (DV / NC) + c % CV];
+    for (int c = 0; c < TC; ++c) acc[r][c] = 0.0f;
 #pragma unroll 2
   for (int j = 0; j < n; ++j) {
     const float w = pw[first + step * j];
@@ -103,7 +103,10 @@ template <int DK, int DV> __device__ __forceinline__ void update_state(float* S,
 #pragma unroll
   for (int r = 0; r < TR; ++r)
 #pragma unroll
-    for (int c = 0; c < TC; ++c) s0[r * (DV + 4) + (c / CV) * (DV / NC) + c % CV] = acc[r][c];
+    for (int c = 0; c < TC; ++c) {
+      float& x = s0[r * (DV + 4) + (c / CV) * (DV / NC) + c % CV];
+      x = fmaf(decay, x, acc[r][c]);
+    }
 }
 
 __device__ __forceinline__ float dot4(float4 a, float4 b, float c) {
@@ -114,11 +117,16 @@ template <int W, bool UP> __device__ __forceinline__ void scores(float* P, const
   const int x = threadIdx.x >> 3, y0 = threadIdx.x & 7;
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
   const float* xr = X + x * (W + 4);
+  for (int k0 = 0; k0 < W; k0 += 32) {
+    float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
-  for (int k = 0; k < W; k += 4) {
-    const float4 a = *reinterpret_cast<const float4*>(xr + k);
+    for (int k = k0; k < k0 + 32; k += 4) {
+      const float4 a = *reinterpret_cast<const float4*>(xr + k);
 #pragma unroll
-    for (int m = 0; m < 4; ++m) acc[m] = dot4(a, *reinterpret_cast<const float4*>(Y + (y0 + 8 * m) * (W + 4) + k), acc[m]);
+      for (int m = 0; m < 4; ++m) sum[m] = dot4(a, *reinterpret_cast<const float4*>(Y + (y0 + 8 * m) * (W + 4) + k), sum[m]);
+    }
+#pragma unroll
+    for (int m = 0; m < 4; ++m) acc[m] += sum[m];
   }
 #pragma unroll
   for (int m = 0; m < 4; ++m) {
@@ -134,44 +142,59 @@ template <int W> struct Own {
   int row, col;
   __device__ __forceinline__ Own(bool strided) : row((threadIdx.x / GROUPS) * ROWS), col((threadIdx.x % GROUPS) * (strided ? 1 : 4)) {}
 };
+template <int R> __device__ __forceinline__ void add_to(float (&acc)[R][4], const float (&sum)[R][4]) {
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[r][c] += sum[r][c];
+}
 // acc += A[row] M  for the [K][N] matrix M (pitch N + 4)
 template <int K, int N> __device__ __forceinline__ void times(float (&acc)[N / 32][4], const float* A, const float* M, const Own<N>& own) {
+  for (int k0 = 0; k0 < K; k0 += 32) {
+    float sum[N / 32][4] = {};
 #pragma unroll 2
-  for (int k = 0; k < K; k += 4) {
-    float4 m[4];
+    for (int k = k0; k < k0 + 32; k += 4) {
+      float4 m[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) m[i] = *reinterpret_cast<const float4*>(M + (k + i) * (N + 4) + own.col);
+      for (int i = 0; i < 4; ++i) m[i] = *reinterpret_cast<const float4*>(M + (k + i) * (N + 4) + own.col);
 #pragma unroll
-    for (int r = 0; r < N / 32; ++r) {
-      const float4 a = *reinterpret_cast<const float4*>(A + (own.row + r) * (K + 4) + k);
-      const float e[4] = {a.x, a.y, a.z, a.w};
+      for (int r = 0; r < N / 32; ++r) {
+        const float4 a = *reinterpret_cast<const float4*>(A + (own.row + r) * (K + 4) + k);
+        const float e[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        acc[r][0] = fmaf(e[i], m[i].x, acc[r][0]); acc[r][1] = fmaf(e[i], m[i].y, acc[r][1]);
-        acc[r][2] = fmaf(e[i], m[i].z, acc[r][2]); acc[r][3] = fmaf(e[i], m[i].w, acc[r][3]);
+        for (int i = 0; i < 4; ++i) {
+          sum[r][0] = fmaf(e[i], m[i].x, sum[r][0]); sum[r][1] = fmaf(e[i], m[i].y, sum[r][1]);
+          sum[r][2] = fmaf(e[i], m[i].z, sum[r][2]); sum[r][3] = fmaf(e[i], m[i].w, sum[r][3]);
+        }
       }
     }
+    add_to<N / 32>(acc, sum);
   }
 }
 // acc += A[row] M^T for the [N][K] matrix M (pitch K + 4), columns N/4 apart
 template <int K, int N> __device__ __forceinline__ void times_t(float (&acc)[N / 32][4], const float* A, const float* M, const Own<N>& own) {
+  for (int k0 = 0; k0 < K; k0 += 32) {
+    float sum[N / 32][4] = {};
 #pragma unroll 2
-  for (int k = 0; k < K; k += 4) {
-    float4 m[4];
+    for (int k = k0; k < k0 + 32; k += 4) {
+      float4 m[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) m[i] = *reinterpret_cast<const float4*>(M + (own.col + i * (N / 4)) * (K + 4) + k);
+      for (int i = 0; i < 4; ++i) m[i] = *reinterpret_cast<const float4*>(M + (own.col + i * (N / 4)) * (K + 4) + k);
 #pragma unroll
-    for (int r = 0; r < N / 32; ++r) {
-      const float4 a = *reinterpret_cast<const float4*>(A + (own.row + r) * (K + 4) + k);
+      for (int r = 0; r < N / 32; ++r) {
+        const float4 a = *reinterpret_cast<const float4*>(A + (own.row + r) * (K + 4) + k);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) acc[r][i] = dot4(a, m[i], acc[r][i]);
+        for (int i = 0; i < 4; ++i) sum[r][i] = dot4(a, m[i], sum[r][i]);
+      }
     }
+    add_to<N / 32>(acc, sum);
   }
 }
 // acc += P[row] M over the causal side of the 32 x 32 tile P (y <= row, or y >= row with UP), M [32][N]
 template <int N, bool STRIDED, bool UP> __device__ __forceinline__ void times_scores(float (&acc)[N / 32][4], const float* P, const float* M,
                                                                                     const Own<N>& own) {
   constexpr int R = N / 32;
+  float sum[R][4] = {};
   const int lo = UP ? own.row & ~3 : 0, hi = UP ? L32 : (own.row + R + 3) & ~3;
   for (int k = lo; k < hi; k += 4) {
     const bool whole = UP ? k >= own.row + R - 1 : k + 3 <= own.row;
@@ -186,12 +209,13 @@ template <int N, bool STRIDED, bool UP> __device__ __forceinline__ void times_sc
         const int row = own.row + r;
         if (whole || (UP ? k + i >= row : k + i <= row)) {
           const float e = P[row * PP + k + i];
-          acc[r][0] = fmaf(e, m.x, acc[r][0]); acc[r][1] = fmaf(e, m.y, acc[r][1]);
-          acc[r][2] = fmaf(e, m.z, acc[r][2]); acc[r][3] = fmaf(e, m.w, acc[r][3]);
+          sum[r][0] = fmaf(e, m.x, sum[r][0]); sum[r][1] = fmaf(e, m.y, sum[r][1]);
+          sum[r][2] = fmaf(e, m.z, sum[r][2]); sum[r][3] = fmaf(e, m.w, sum[r][3]);
         }
       }
     }
   }
+  add_to<R>(acc, sum);
 }
 template <int N> __device__ __forceinline__ void scale_rows(float (&acc)[N / 32][4], const Own<N>& own, const float* pw, int first, int step, int n) {
 #pragma unroll
