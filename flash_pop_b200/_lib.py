@@ -165,6 +165,8 @@ _SIGNATURES = {
     "fpb_layernorm_bwd": [ctypes.c_int64, ctypes.c_int32, ctypes.c_int32, ctypes.c_float, ctypes.c_void_p, ctypes.c_int64,
                           ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                           ctypes.c_void_p],
+    "fpb_column_sums": [ctypes.c_int64, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p,
+                        ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p],
     "fpb_cross_entropy_fwd": [ctypes.c_int64, ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p,
                               ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p],
     "fpb_cross_entropy_bwd": [ctypes.c_int64, ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p,
@@ -236,7 +238,7 @@ def lib() -> ctypes.CDLL:
 # entry points of the C ABI that the host-side extension calls, in the order of its table
 _NATIVE_ENTRIES = ("fpb_retention_fwd", "fpb_retention_bwd", "fpb_pop_retention_fwd", "fpb_pop_retention_bwd", "fpb_pop_suffix_fwd",
                    "fpb_pop_suffix_bwd", "fpb_retention_step", "fpb_workspace_bytes", "fpb_rotary", "fpb_groupnorm_gate_fwd",
-                   "fpb_groupnorm_gate_bwd", "fpb_layernorm_fwd", "fpb_layernorm_bwd")
+                   "fpb_groupnorm_gate_bwd", "fpb_layernorm_fwd", "fpb_layernorm_bwd", "fpb_column_sums")
 _native = None
 _native_bound: Optional[ctypes.CDLL] = None
 

@@ -566,6 +566,19 @@ int fpb_layernorm_bwd(int64_t rows, int32_t d, int32_t dtype, float eps, const v
   return finish_launches(1, -1);
 }
 
+int fpb_column_sums(int64_t rows, int64_t n, const void* g, int64_t g_stride, const void* a, void* d_a, void* scratch, void* sums,
+                    fpb_stream_t stream) {
+  if (rows <= 0 || n <= 0 || n % 64 || n > FPB_COLUMN_SUMS_SCRATCH / 4) return FPB_ERR_BAD_SHAPE;
+  if (!g || !sums || !scratch || (a && !d_a)) return FPB_ERR_NULL_POINTER;
+  if ((rows > 1 && g_stride < n) || g_stride % 8 || (uintptr_t)g % 16 || (uintptr_t)a % 16 || (uintptr_t)d_a % 16 || (uintptr_t)sums % 2 ||
+      (uintptr_t)scratch % 16)
+    return FPB_ERR_BAD_STRIDE;
+  FPB_TRY(check_device());
+  const int r = launch_column_sums(rows, n, g, g_stride, a, d_a, (float*)scratch, sums, (cudaStream_t)stream);
+  const int f = finish_launches(2, -1);
+  return r != FPB_OK ? r : f;
+}
+
 namespace {
 // a (mod_rows, d) operand shared by rows_per_mod consecutive rows of the activations
 int check_mod(int64_t rows, int32_t d, int32_t dtype, const void* ptr, int64_t mod_stride, int64_t rows_per_mod) {

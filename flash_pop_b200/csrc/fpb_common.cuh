@@ -75,6 +75,10 @@ int check_decoder_token(const fpb_token_dims& d, const fpb_decoder_layer* layers
 int launch_decoder_token(const fpb_token_dims& d, const fpb_decoder_layer* layers, const float* gamma, const void* x, int64_t x_stride,
                          void* y, int64_t y_stride, cudaStream_t stream, int* n_launched);
 
+// Column sums of a (rows, n) gradient, after the backward of x sigmoid(x) where `a` is given (linear_grads.cu).
+int launch_column_sums(int64_t rows, int64_t n, const void* g, int64_t g_stride, const void* a, void* out, float* partial, void* sums,
+                       cudaStream_t stream);
+
 // Fused elementwise passes around the operator (layer_fused.cu).
 int launch_rotary(int in_dtype, int out_dtype, int B, int T, int H, int d, bool conjugate, const float* phasors,
                   int64_t phasor_stride_b, const SeqView in[2], const SeqView out[2], int n_tensors, cudaStream_t stream);

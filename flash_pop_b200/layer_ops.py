@@ -361,3 +361,119 @@ def cross_entropy(logits: Tensor, targets: Tensor) -> Tensor:
     safe = torch.where(valid, targets, torch.zeros_like(targets))
     per_row = torch.nn.functional.cross_entropy(logits.float(), safe, reduction="none")
     return (per_row * valid.to(per_row.dtype)).sum() / max(logits.size(0), 1)
+
+
+# ---- linear layers of a decoder layer in training -------------------------------------------------------------------
+def observed() -> bool:
+    """Something wants to see the individual operations: autocast, a dispatch or function mode, tracing, forward-mode
+    gradients, a function transform, a hook on every module."""
+    m = torch.nn.modules.module
+    return (torch.is_autocast_enabled("cuda") or torch._C._len_torch_dispatch_stack() > 0 or torch._C._len_torch_function_stack() > 0
+            or torch.autograd.forward_ad._current_level >= 0 or torch.compiler.is_compiling() or torch.jit.is_tracing()
+            or torch._C._functorch.maybe_current_level() is not None
+            or bool(m._global_forward_hooks or m._global_forward_pre_hooks or m._global_backward_hooks or m._global_backward_pre_hooks))
+
+
+def linears_supported(x: Tensor, *linears) -> bool:
+    """Whether a gradient is being recorded through plain bf16 ``nn.Linear`` modules that nothing is attached to, on rows
+    the column-sum kernel reads."""
+    if not (torch.is_grad_enabled() and type(x) is Tensor and x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and x.numel() > 0):
+        return False
+    for m in linears:
+        if type(m) is not torch.nn.Linear:
+            return False
+        d = m.__dict__
+        if d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"] or "forward" in d:
+            return False
+        w, b = d["_parameters"].get("weight"), d["_parameters"].get("bias")
+        if w is None or b is None or w.dtype != torch.bfloat16 or b.dtype != torch.bfloat16 or not (w.requires_grad and b.requires_grad):
+            return False
+        if w.device != x.device or m.out_features % 64 or type(w) is not torch.nn.Parameter or type(b) is not torch.nn.Parameter:
+            return False
+    return not observed()
+
+
+def _bias_grad(g: Tensor) -> Tensor:
+    """Sum over all rows: the library's kernel, or the framework's where a graph of this backward is wanted or the
+    gradient's layout is not the ordinary one."""
+    if not torch.is_grad_enabled():
+        fast = _lib.result(_lib.native().column_sums(g, None))
+        if fast is not None:
+            return fast[0]
+    return g.sum(dim=tuple(range(g.dim() - 1)))
+
+
+def _rows2(t: Tensor) -> Tensor:
+    return t.reshape(-1, t.size(-1))
+
+
+class SharedInputLinears(torch.autograd.Function):
+    """``tuple(F.linear(x, w, b) for w, b in pairs)``: the gradients of x meet in the matrix products' accumulation instead of
+    additions of their own, and the biases' gradients are column sums of the library."""
+
+    @staticmethod
+    def forward(ctx, x, *params):
+        ctx.save_for_backward(x, *params[0::2])
+        ctx.set_materialize_grads(False)
+        return tuple(torch.nn.functional.linear(x, w, b) for w, b in zip(params[0::2], params[1::2]))
+
+    @staticmethod
+    def backward(ctx, *grads):
+        x, *weights = ctx.saved_tensors
+        x2, dx, out = _rows2(x), None, []
+        for i, (g, w) in enumerate(zip(grads, weights)):
+            if g is None:
+                out += (None, None)
+                continue
+            need_w, need_b = ctx.needs_input_grad[1 + 2 * i], ctx.needs_input_grad[2 + 2 * i]
+            g2 = _rows2(g)
+            db = _bias_grad(g) if need_b else None         # (first: it binds the device to this thread, which cuBLAS wants done)
+            if ctx.needs_input_grad[0]:
+                # (in place where no graph of this backward is wanted: out of place the sum is copied first)
+                dx = g2.mm(w) if dx is None else torch.addmm(dx, g2, w) if torch.is_grad_enabled() else dx.addmm_(g2, w)
+            out += (g2.t().mm(x2) if need_w else None, db)
+        return (None if dx is None else dx.view(x.shape), *out)
+
+
+def linear_group(x: Tensor, *linears) -> Tuple[Tensor, ...]:
+    """``tuple(m(x) for m in linears)``."""
+    if linears_supported(x, *linears):
+        return SharedInputLinears.apply(x, *(p for m in linears for p in (m.weight, m.bias)))
+    return tuple(m(x) for m in linears)
+
+
+class SwishFeedForward(torch.autograd.Function):
+    """``F.linear(F.silu(F.linear(x, w1, b1)), w2, b2)``; backward takes the gradient through the activation and sums its
+    columns (the first bias's gradient) in one pass."""
+
+    @staticmethod
+    def forward(ctx, x, w1, b1, w2, b2):
+        a = torch.nn.functional.linear(x, w1, b1)
+        h = torch.nn.functional.silu(a)
+        ctx.save_for_backward(x, a, h, w1, w2, b1, b2)
+        return torch.nn.functional.linear(h, w2, b2)
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, a, h, w1, w2, b1, b2 = ctx.saved_tensors
+        need = ctx.needs_input_grad
+        if torch.is_grad_enabled():          # a graph of this backward is wanted: through the framework's own operations
+            inputs = (x, w1, b1, w2, b2)
+            y = torch.nn.functional.linear(torch.nn.functional.silu(torch.nn.functional.linear(x, w1, b1)), w2, b2)
+            got = iter(torch.autograd.grad(y, [t for t, n in zip(inputs, need) if n], dy, create_graph=True))
+            return tuple(next(got) if n else None for n in need)
+        dy2 = _rows2(dy)
+        db2 = _bias_grad(dy) if need[4] else None      # (first: it binds the device to this thread, which cuBLAS wants done)
+        dw2 = dy2.t().mm(_rows2(h)) if need[3] else None
+        dh = dy2.mm(w2).view(a.shape)
+        fast = _lib.result(_lib.native().column_sums(dh, a))
+        if fast is not None:
+            db1, da = fast
+        else:
+            s = torch.sigmoid(a.float())
+            da = (dh.float() * s * (1 + a.float() * (1 - s))).to(dh.dtype)
+            db1 = _bias_grad(da)
+        da2 = _rows2(da)
+        dw1 = da2.t().mm(_rows2(x)) if need[1] else None
+        dx = da2.mm(w1).view(x.shape) if need[0] else None
+        return dx, dw1, db1 if need[2] else None, dw2, db2

@@ -36,6 +36,7 @@ struct Entry {
   decltype(&fpb_groupnorm_gate_bwd) gate_bwd;
   decltype(&fpb_layernorm_fwd) norm_fwd;
   decltype(&fpb_layernorm_bwd) norm_bwd;
+  decltype(&fpb_column_sums) column_sums;
 } entry;
 constexpr int ENTRIES = sizeof(Entry) / sizeof(void*), MAX_HEADS = 256;
 
@@ -459,6 +460,27 @@ PyObject* norm_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+// column_sums(g (..., n), a or None) -> (sums (n), d_a or None): all contiguous bf16
+PyObject* column_sums(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded(n, 2, [&]() -> PyObject* {
+    const at::Tensor g = tensor(a[0]), act = maybe(a[1]);
+    NEED(g.scalar_type() == at::kBFloat16 && g.dim() >= 1 && g.is_contiguous() && g.size(-1) % 64 == 0 && (uintptr_t)g.data_ptr() % 16 == 0);
+    if (act.defined())
+      NEED(act.scalar_type() == at::kBFloat16 && act.is_contiguous() && act.sizes() == g.sizes() && act.device() == g.device() &&
+           (uintptr_t)act.data_ptr() % 16 == 0);
+    const int64_t cols = g.size(-1), rows = g.numel() / cols;
+    NEED(cols <= FPB_COLUMN_SUMS_SCRATCH / 4);
+    Place here(g);
+    const at::Tensor scratch = make({FPB_COLUMN_SUMS_SCRATCH}, g, at::kByte);
+    const at::Tensor sums = make({cols}, g, at::kBFloat16), d_a = act.defined() ? make(g.sizes(), g, at::kBFloat16) : at::Tensor();
+    const int r = unlocked([&] {
+      return entry.column_sums(rows, cols, g.data_ptr(), cols, act.defined() ? act.data_ptr() : nullptr, d_a.defined() ? d_a.data_ptr() : nullptr,
+                               scratch.data_ptr(), sums.data_ptr(), here.stream);
+    });
+    return r ? PyLong_FromLong(r) : tuple_of({sums, d_a});
+  });
+}
+
 // address(t, dtype, align, device_index, n0, n1) -> address of a contiguous parameter of that shape (n1 = 0: one dimension), or None
 PyObject* address(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded(n, 6, [&]() -> PyObject* {
@@ -486,7 +508,7 @@ PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 #define FAST(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {FAST(step), FAST(forward), FAST(backward), FAST(suffix_forward), FAST(suffix_backward), FAST(rotary), FAST(gate_forward),
-                         FAST(gate_backward), FAST(norm_forward), FAST(norm_backward), FAST(address), FAST(bind), {nullptr, nullptr, 0, nullptr}};
+                         FAST(gate_backward), FAST(norm_forward), FAST(norm_backward), FAST(column_sums), FAST(address), FAST(bind), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "fpb_fast_calls", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

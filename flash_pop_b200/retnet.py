@@ -26,7 +26,7 @@ import torch.nn.functional as F
 from torch import Tensor
 
 from flash_pop_b200.fused_retention import cuda_core_kernels, fused_chunk_retention, retention_step
-from flash_pop_b200.layer_ops import groupnorm_gate, groupnorm_gate_supported, norm_in_fp32
+from flash_pop_b200.layer_ops import SwishFeedForward, groupnorm_gate, groupnorm_gate_supported, linear_group, linears_supported, norm_in_fp32
 from flash_pop_b200.recurrent_state import RecurrentState
 from flash_pop_b200.token_stack import decoder_token
 from flash_pop_b200.xpos_emb import XPos
@@ -144,18 +144,20 @@ class MultiScaleRetention(nn.Module):
         with cuda_core_kernels():
             return fused_chunk_retention(q, k, v, prev_state, self.head_decays)
 
-    def _gate_and_project(self, retention: Tensor, x: Tensor) -> Tensor:
-        """GroupNorm over each head of each token (fp32), swish gate, output projection."""
+    def _gate_and_project(self, retention: Tensor, x: Tensor, z: Optional[Tensor] = None) -> Tensor:
+        """GroupNorm over each head of each token (fp32), swish gate, output projection.  z: ``g_proj(x)``, where the
+        caller has it."""
         shape = retention.shape[:-2]
         dropping = self.dropout > 0 and self.training
-        z = self.g_proj(x)
+        if z is None:
+            z = self.g_proj(x)
         o4 = retention.reshape(-1, 1, self.num_heads, self.head_dim_v) if retention.dim() == 3 else retention
         if retention.dim() in (3, 4) and not dropping and z.dtype == retention.dtype:
             z4 = z.reshape(o4.shape)
             if groupnorm_gate_supported(o4, z4):
                 swish = self.activation is F.silu
                 gated = groupnorm_gate(o4, z4 if swish else self.activation(z4), self.group_norm.eps, swish)
-                return self.out_proj(gated.reshape(*shape, self.embed_dim))
+                return linear_group(gated.reshape(*shape, self.embed_dim), self.out_proj)[0]
         flat = retention.reshape(-1, self.embed_dim)
         flat = F.dropout(flat, p=self.dropout, training=self.training)
         flat = self.group_norm(flat.float()).to(dtype=x.dtype)
@@ -164,9 +166,12 @@ class MultiScaleRetention(nn.Module):
     def _retention_chunkwise(self, x: Tensor, start_idx: Union[int, torch.LongTensor], prev_state: Optional[Tensor] = None,
                              retention_kernel: Optional[Callable] = None, xpos_embedder: Optional[XPos] = None):
         """x: (B, T, H*dv).  Returns the layer output (B, T, H*dv) and whatever state(s) the kernel returns."""
-        q = _split_heads(self.q_proj(x).to(dtype=x.dtype), self.num_heads)
-        k = _split_heads(self.k_proj(x).to(dtype=x.dtype), self.num_heads)
-        v = _split_heads(self.v_proj(x).to(dtype=x.dtype), self.num_heads)
+        gate = {}
+        if type(self)._gate_and_project is MultiScaleRetention._gate_and_project and "_gate_and_project" not in self.__dict__:
+            q, k, v, gate["z"] = linear_group(x, self.q_proj, self.k_proj, self.v_proj, self.g_proj)
+        else:
+            q, k, v = linear_group(x, self.q_proj, self.k_proj, self.v_proj)
+        q, k, v = (_split_heads(t.to(dtype=x.dtype), self.num_heads) for t in (q, k, v))
         if self.relative_position:
             q, k = (xpos_embedder or self.xpos_embedder)(q, k, start_idx)
         if prev_state is None:
@@ -174,7 +179,7 @@ class MultiScaleRetention(nn.Module):
         kernel = retention_kernel or self._compute_chunkwise_retention_kernel
         retention, state = kernel(q.bfloat16(), k.bfloat16(), v.bfloat16(), prev_state.bfloat16())
         retention, state = retention.to(dtype=x.dtype), state.to(dtype=x.dtype)
-        return self._gate_and_project(retention, x).to(dtype=x.dtype), state
+        return self._gate_and_project(retention, x, **gate).to(dtype=x.dtype), state
 
     def forward_chunkwise(self, x: Tensor, start_idx: Union[int, torch.LongTensor], prev_state: Optional[Tensor] = None):
         return self._retention_chunkwise(x, start_idx, prev_state)
@@ -242,6 +247,10 @@ class RetNetDecoderLayer(nn.Module):
             nn.init.constant_(lin.bias, 0)
 
     def _feedforward_block(self, x: Tensor) -> Tensor:
+        drop = self.dropout
+        if (self.activation is F.silu and type(drop) is nn.Dropout and (drop.p == 0 or not drop.training) and not drop._forward_hooks
+                and not drop._forward_pre_hooks and linears_supported(x, self.linear1, self.linear2)):
+            return SwishFeedForward.apply(x, self.linear1.weight, self.linear1.bias, self.linear2.weight, self.linear2.bias)
         x = self.dropout(self.activation(self.linear1(x)))
         return self.dropout(self.linear2(x))
 

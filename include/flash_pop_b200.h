@@ -237,6 +237,17 @@ int fpb_decoder_token(const fpb_token_dims* dims, const fpb_decoder_layer* layer
                       void* y, int64_t y_stride, fpb_stream_t stream);
 
 /*
+ * Bias gradients of linear layers: sums[c] = sum over the rows of g[r, c], fp32 sums, bf16 in and out.  n a multiple of 64,
+ * rows 16-byte aligned.  With `a` (rows, n) contiguous, g is the gradient of y = a sigmoid(a): it is first taken back through
+ * the activation, into d_a (rows, n) contiguous, and d_a's columns are what is summed.  (The feed-forward of
+ * flash_pop/retnet.py:247-268; the reference leaves both to the framework.)  `scratch`: FPB_COLUMN_SUMS_SCRATCH device bytes,
+ * 16-byte aligned, used during the call only; n at most a quarter of that.
+ */
+#define FPB_COLUMN_SUMS_SCRATCH (592 * 256 * 4)
+int fpb_column_sums(int64_t rows, int64_t n, const void* g, int64_t g_stride, const void* a, void* d_a, void* scratch, void* sums,
+                    fpb_stream_t stream);
+
+/*
  * The two elementwise passes of a retention layer either side of the operator, each as one streaming kernel
  * (fp32 arithmetic).  They replace PyTorch expressions of the reference rather than kernels of its own.
  *
