@@ -254,6 +254,20 @@ using namespace fpb;
 
 #define FPB_TRY(expr) do { const int _s = (expr); if (_s != FPB_OK) return _s; } while (0)
 
+namespace {
+// What decides whether fpb_retention_fwd_static takes a shape: the scratch of pieces of at least 512 tokens.  Within the
+// built-in scratch a call is split as far as that allows.  (fp32 calls are taken whatever their size.)
+int64_t static_split_bytes(const fpb_dims& d) {
+  if (d.dtype != FPB_BF16 || d.B <= 0 || d.H <= 0) return 0;
+  const int64_t units = (int64_t)d.B * d.H, slots = (int64_t)sm_count() * ((d.dk <= 64 || d.dv <= 64) ? 2 : 1);
+  int64_t n = units * 2 > sm_count() ? 1 : slots / units;
+  n = n < d.T / 512 ? n : d.T / 512;
+  if (n < 2) return 0;
+  const int64_t len = ((d.T + n - 1) / n + 63) / 64 * 64, count = (d.T + len - 1) / len;
+  return count < 2 ? 0 : units * count * d.dk * d.dv * 4;
+}
+}  // namespace
+
 extern "C" {
 
 int fpb_retention_fwd(const fpb_dims* dims, const fpb_seq* q, const fpb_seq* k, const fpb_seq* v,
@@ -277,9 +291,7 @@ int fpb_retention_fwd_static(const fpb_dims* dims, const fpb_seq* q, const fpb_s
   FPB_TRY(check_seq(c, v, c.dv, c.B)); FPB_TRY(check_seq(c, o, c.dv, c.B));
   FPB_TRY(check_state(s0, c)); FPB_TRY(check_state(s_out, c));
   FPB_TRY(check_device());
-  // a shape whose full split needs more than the built-in scratch holds is refused rather than split less (fp32 calls,
-  // whose kernels take any amount, split as far as it goes)
-  if (dims->dtype == FPB_BF16 && fpb_workspace_bytes(dims) > (int64_t)FPB_STATIC_SCRATCH_BYTES) return FPB_ERR_TOO_LARGE;
+  if (static_split_bytes(*dims) > (int64_t)FPB_STATIC_SCRATCH_BYTES) return FPB_ERR_TOO_LARGE;
   float* scratch = static_scratch_ptr();
   if (!scratch) { tl_last_cuda_error = (int)cudaErrorInvalidSymbol; return FPB_ERR_LAUNCH; }
   c.scratch = scratch;

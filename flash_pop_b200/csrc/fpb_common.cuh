@@ -124,6 +124,7 @@ struct Segments {
 // segment start must be a multiple of; state_floats = dk * dv; scratch holds B*H*n*state_floats floats.
 Segments choose_segments(long long units, int ctas_per_sm, int T, int align, long long batch_heads, long long state_floats,
                          long long scratch_bytes, int B);
+int sm_count();              // of the current device
 // Start values of the segments from the local end values of all but the piece reached last: in place over `seg`
 // (B, H, n, dk, dv) fp32.
 //   forward : A_0 = start, A_{s+1} = gamma^len_s A_s + E_s ; seg[s] <- A_s

@@ -71,6 +71,8 @@ __global__ void __launch_bounds__(256) segment_combine_kernel(const __grid_const
   }
 }
 
+}  // namespace
+
 int sm_count() {
   static std::atomic<int> cache[64];
   int dev = 0;
@@ -83,9 +85,19 @@ int sm_count() {
   return n;
 }
 
-}  // namespace
+constexpr int kLongPiece = 512;          // tokens
 
-constexpr int kMinSegmentTokens = 512;   // a piece shorter than 8 chunks does not pay for its pipeline fill
+// What a walk costs, in tenths of a microsecond (fitted to one B200, 4 to 32 heads in all, d = 64 and 128, T = 300 to 5000):
+// whole, 60 and 15.5 a chunk of its sequence; in pieces - state pass, scan and walk, three set-ups - 160 and 26 a chunk of a
+// piece.  The two launches more are worth 6 us of the host's time.  Both sides measured (forward, us): 8 heads, T = 1000,
+// d = 128 whole 30.8, 8 pieces 22.7; 4 heads, T = 3000 in 5 pieces 41.1, in 24 26.3; but 16 heads, T = 600 whole 20.7, 4
+// pieces 24.7, 8 heads, T = 300 whole 13.7, 2 pieces 22.7, and 32 heads, T = 777, d = 64 whole 22.8, 7 pieces 18.6, which a
+// training call of 100 us of host work pays with 10 us.  (Pieces of at least 512 tokens, the rule before the launches were
+// chained, left the first two at 30.8 and 41.1.)
+static bool pieces_pay(int T, int seg_len) {
+  const long long chunks = (T + 63) / 64, per_piece = (seg_len + 63) / 64;
+  return 10 * (160 + 26 * per_piece + 60) < 10 * 60 + 155 * chunks;
+}
 
 Segments choose_segments(long long units, int ctas_per_sm, int T, int align, long long batch_heads, long long state_floats,
                          long long scratch_bytes, int B) {
@@ -96,20 +108,21 @@ Segments choose_segments(long long units, int ctas_per_sm, int T, int align, lon
   const long long sms = sm_count();
   const long long slots = sms * ctas_per_sm;
   if (units <= 0 || units * 2 > sms || align <= 0) return none;
-  const int min_len = ((kMinSegmentTokens + align - 1) / align) * align;
-  long long n = slots / units;
-  if (n > T / min_len) n = T / min_len;
+  long long most = slots / units;
   if (scratch_bytes > 0) {                                               // 0: the caller only asks how far a split would go
     const long long fit = scratch_bytes / (batch_heads * state_floats * 4);
-    if (n > fit) n = fit;
+    if (most > fit) most = fit;
   }
-  if (B > 0 && n > 65535 / B) n = 65535 / B;                             // grid.z = batch x pieces
-  if (n < 2) return none;
-  const long long per = (T + n - 1) / n;
-  const int seg_len = (int)((per + align - 1) / align) * align;
-  const int count = (T + seg_len - 1) / seg_len;
-  if (count < 2) return none;
-  return Segments{count, seg_len};
+  if (B > 0 && most > 65535 / B) most = 65535 / B;                       // grid.z = batch x pieces
+  auto cut = [&](long long shortest) {                                   // into as many pieces as allowed, each at least that long
+    const long long n = most < T / shortest ? most : T / shortest;
+    if (n < 2) return none;
+    const int seg_len = (int)(((T + n - 1) / n + align - 1) / align) * align, count = (T + seg_len - 1) / seg_len;
+    return count < 2 ? none : Segments{count, seg_len};
+  };
+  const Segments fine = cut(align);
+  if (fine.n > 1 && pieces_pay(T, fine.seg_len)) return fine;
+  return cut(((kLongPiece + align - 1) / align) * align);                // pieces this long always paid
 }
 
 int launch_segment_combine(float* seg, Segments sg, int B, int T, int H, int dk, int dv, const float* gamma, bool reverse,
