@@ -53,6 +53,7 @@ struct BwdParams {
   void* sfx_blocks; int32_t sfx_M, sfx_N;        // suffix calls: gradients of the start states taken from block states
   int32_t sfx_G;                                 // suffixes one CTA walks back to back as one sequence (>= 1)
   int32_t T, H, dk, dv, block_size, n_blocks;
+  int32_t half0, dk_add;                         // dv = 2 DV: first half of this launch; dK is added to the output
   int32_t state_f32;
   int32_t n_seg, seg_len;                        // T-segments (segment_scan.cu): blockIdx.z = batch * n_seg + segment
   const float* seg_states;                       // fp32 (B, H, n_seg, dk, dv): G after the last token of each segment
@@ -129,10 +130,9 @@ __global__ void __launch_bounds__(BCfg<DK, DV>::NTHREADS, 1) bwd_fused_kernel(co
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int h = blockIdx.y;
-  // dv = 2 DV: blockIdx.x is the half of dv this CTA takes.  dV and the G columns of the half are complete; dK is a
-  // partial sum over the half's columns, which TMA adds to the (zeroed) output.
-  const int vcol = (int)blockIdx.x * DV;
-  const bool dv_split = gridDim.x > 1;
+  // dv = 2 DV: blockIdx.x + half0 is the half of dv this CTA takes.  dV and the G columns of the half are complete; dK is a
+  // partial sum over the half's columns, which TMA adds to the output (zeroed, or stored by the launch of the first half).
+  const int vcol = ((int)blockIdx.x + p.half0) * DV;
   const int b = p.n_seg > 1 ? (int)blockIdx.z / p.n_seg : (int)blockIdx.z;
   const int seg = p.n_seg > 1 ? (int)blockIdx.z % p.n_seg : 0;
   // this CTA walks tokens [t0, t_end) of the sequence; chunk positions are absolute (t0 is a chunk and block multiple)
@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(BCfg<DK, DV>::NTHREADS, 1) bwd_fused_kernel(co
         if (t == 0) {
 #pragma unroll
           for (int cb = 0; cb < DV / 64; ++cb) tma_store_4d(&p.map_dv, sbase + G::OFF_OUTV + cb * 8192, vcol + cb * 64, ck.a, h, b);
-          if (dv_split) {
+          if (p.dk_add) {
 #pragma unroll
             for (int cb = 0; cb < DK / 64; ++cb) tma_reduce_add_4d(&p.map_dk, sbase + G::OFF_OUTK + cb * 8192, cb * 64, ck.a, h, b);
           } else {
@@ -824,8 +824,11 @@ int launch_bwd_fused(const UmmaBwdArgs& a, cudaStream_t stream, int* n_launched)
   p.trace = debug_trace_ptr();
   if (!p.status) return FPB_ERR_LAUNCH;
   for (int h = 0; h < H; ++h) p.log2g[h] = (float)std::log2((double)a.gamma[h]);
-  const dim3 grid(dv_halves ? 2 : 1, H, B * sg.n);
-  if (dv_halves) {
+  const bool apart = dv_halves && sg.n == 1 && halves_apart((long long)B * H);
+  const dim3 grid(dv_halves && !apart ? 2 : 1, H, B * sg.n);
+  p.half0 = 0;
+  p.dk_add = dv_halves && !apart ? 1 : 0;
+  if (p.dk_add) {
     launch_zero_seq(dK, B, T, H, a.dk, stream);
     ++*n_launched;
   }
@@ -834,6 +837,11 @@ int launch_bwd_fused(const UmmaBwdArgs& a, cudaStream_t stream, int* n_launched)
   if (a.dk == DK_ && tile_dv == DV_) r = a.state_f32 ? launch_fused_t<DK_, DV_, true>(p, grid, stream) : launch_fused_t<DK_, DV_, false>(p, grid, stream)
   r = FPB_ERR_BAD_SHAPE;
   FPB_FUSED_CASE(128, 128); FPB_FUSED_CASE(64, 64); FPB_FUSED_CASE(64, 128); FPB_FUSED_CASE(128, 64);
+  if (r == FPB_OK && apart) {
+    ++*n_launched;
+    p.half0 = 1; p.dk_add = 1;
+    FPB_FUSED_CASE(128, 128);
+  }
 #undef FPB_FUSED_CASE
   if (r == FPB_OK) ++*n_launched;
   return r;

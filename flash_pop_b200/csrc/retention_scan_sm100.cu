@@ -97,7 +97,9 @@ struct ScanParams {
                                  // emitted from inside full chunks (forward walk, 64 x 64 tiles, see EMIT below)
   int32_t state_f32;             // element type of s0, s_out, block states / gradients and suffix start states
   int32_t col_split;             // MODE_DQ walks only: the tiles cut dv (columns of the state) instead of dk, so each CTA's
-                                 // output tile is a partial sum over its dv columns; TMA adds it to `out` (zeroed before)
+                                 // output tile is a partial sum over its dv columns: 1 - TMA adds it to `out`; 2 - stored,
+                                 // the launch of the other tile adds to it
+  int32_t tile0;                 // first tile of this launch
   int32_t n_seg, seg_len;        // T-segments: blockIdx.z = batch * n_seg + segment, segment s covers tokens [s * seg_len, ...)
   float* seg_states;             // fp32 (B, H, n_seg, dk, dv): start values of the segments (local end values in a STATE_ONLY pass)
   WalkTuning tune;
@@ -206,7 +208,7 @@ scan_kernel(const __grid_constant__ ScanParams p) {
 
   if (SO) grid_dep_release();                          // the scan over the segments may be set up
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tile = blockIdx.x, h = blockIdx.y;
+  const int tile = blockIdx.x + p.tile0, h = blockIdx.y;
   // (a STATE_ONLY pass covers all pieces but the one the walk reaches last - the last one forward, the first one in
   // reverse - whose end value nobody needs ahead of time: the walk proper produces it)
   const int nz = SO ? p.n_seg - 1 : p.n_seg;
@@ -658,7 +660,7 @@ FPB_UNROLL_MMA
         if (!FPB_ABL(64)) fence_async_smem();
         __syncwarp();
         if (lane == 0 && ck.a + wrow0 < p.T) {
-          if (MODE == MODE_DQ && p.col_split) {
+          if (MODE == MODE_DQ && p.col_split == 1) {
 #pragma unroll
             for (int cb = 0; cb < G::NOUT / 64; ++cb)
               tma_reduce_add_4d(&p.map_out, sbase + G::OFF_OUT + cb * 8192 + wrow0 * 128, ocol0 + cb * 64, ck.a + wrow0, h, b);
@@ -1246,7 +1248,8 @@ constexpr int64_t kMaxJoinedTokens = 1 << 30;   // token positions are 32-bit
 int gcd_int(int a, int b) { while (b) { const int t = a % b; a = b; b = t; } return a; }
 
 // One launch of the kernel: the walk itself, or (state_only) the local end values of its T-segments.
-int launch_one(const PassArgs& a, Segments sg, bool state_only, cudaStream_t stream) {
+// `half`: one tile of a walk that cuts dv, by itself - 0 stores its partial result, 1 adds to it; -1: all tiles.
+int launch_one(const PassArgs& a, Segments sg, bool state_only, cudaStream_t stream, int half = -1) {
   const int mode = state_only ? MODE_FWD : a.mode;
   const int xw = mode == MODE_FWD ? a.dk : a.dv, ow = mode == MODE_FWD ? a.dv : a.dk;
   const int B = a.B, T = a.T, H = a.H, dk = a.dk, dv = a.dv;
@@ -1293,8 +1296,9 @@ int launch_one(const PassArgs& a, Segments sg, bool state_only, cudaStream_t str
   if (!p.status) return FPB_ERR_LAUNCH;
   for (int h = 0; h < H; ++h) p.log2g[h] = (float)std::log2((double)a.gamma[h]);
 
-  p.col_split = t.col_split ? 1 : 0;
-  const dim3 grid(t.tiles, H, Bk * (state_only ? sg.n - 1 : sg.n));
+  p.col_split = t.col_split ? (half == 0 ? 2 : 1) : 0;
+  p.tile0 = half > 0 ? half : 0;
+  const dim3 grid(half < 0 ? t.tiles : 1, H, Bk * (state_only ? sg.n - 1 : sg.n));
 #define FPB_SCAN_CASE(MODE_, R_, CC_) \
   if (mode == MODE_ && t.R == R_ && t.CC == CC_) return launch_scan<MODE_, R_, CC_>(p, a.rev, state_only, grid, stream)
   FPB_SCAN_CASE(MODE_FWD, 128, 128); FPB_SCAN_CASE(MODE_FWD, 128, 64); FPB_SCAN_CASE(MODE_FWD, 64, 64);
@@ -1321,6 +1325,12 @@ int launch_pass(const PassArgs& a, cudaStream_t stream, int* n_launched) {
     *n_launched += 2;
   }
   if (tiling_of(a.mode, a.dk, a.dv, col_split_ok(a.mode, a.block_size, a.sfx)).col_split) {
+    if (sg.n == 1 && halves_apart((long long)a.B * a.H)) {
+      if ((r = launch_one(a, sg, false, stream, 0)) != FPB_OK) return r;
+      if ((r = launch_one(a, sg, false, stream, 1)) != FPB_OK) return r;
+      *n_launched += 2;
+      return FPB_OK;
+    }
     launch_zero_seq(a.out, a.B, a.T, a.H, a.mode == MODE_FWD ? a.dv : a.dk, stream);   // the tiles' partial results are added to it
     ++*n_launched;
   }
@@ -1334,6 +1344,14 @@ int launch_pass(const PassArgs& a, cudaStream_t stream, int* n_launched) {
 long long* debug_trace_ptr() { return g_trace; }
 const WalkTuning& walk_tuning() { return g_tuning; }
 bool segments_enabled() { return g_segments != 0; }
+// The two halves of dv as launches of their own, where that takes no more waves of one CTA an SM than one launch of both:
+// the first then stores its partial results and only the second adds, so the zero fill of the output goes (81 us of 537 MB
+// each for dQ and dK at B = 4, H = 32, T = 16384; reading K and Q twice gives part of it back: the whole training call 3582 ->
+// 3540 us).  Same results: adding to a zero is exact.
+bool halves_apart(long long heads) {
+  const long long sms = sm_count_cached(), both = (2 * heads + sms - 1) / sms;
+  return heads * 2 > sms && 2 * ((heads + sms - 1) / sms) <= both;
+}
 bool col_split_enabled() { return g_col_split != 0 && g_tile_pref != 0; }
 void launch_zero_seq(const SeqView& v, int B, int T, int H, int d, cudaStream_t stream) {
   if (B <= 0 || T <= 0) return;

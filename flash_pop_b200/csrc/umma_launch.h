@@ -43,6 +43,8 @@ int launch_segment_states(SeqView k, SeqView v, bool rev, const void* block_grad
 bool segments_enabled();
 // dv = 256: the gradient walks cut dv into 128-wide tiles whose partial results TMA adds to a zeroed output
 bool col_split_enabled();
+// whether the two halves of dv = 256 run as two launches; `heads` = batch rows x heads
+bool halves_apart(long long heads);
 // zeros over the (B, T, H, d) bf16 elements of a strided view (d a multiple of 8, 16-byte aligned rows)
 void launch_zero_seq(const SeqView& v, int B, int T, int H, int d, cudaStream_t stream);
 // How many consecutive suffixes one CTA walks as one sequence; `units` = heads x tiles, each with all `suffixes`.
