@@ -366,12 +366,25 @@ def cross_entropy(logits: Tensor, targets: Tensor) -> Tensor:
 # ---- linear layers of a decoder layer in training -------------------------------------------------------------------
 def observed() -> bool:
     """Something wants to see the individual operations: autocast, a dispatch or function mode, tracing, forward-mode
-    gradients, a function transform, a hook on every module."""
-    m = torch.nn.modules.module
-    return (torch.is_autocast_enabled("cuda") or torch._C._len_torch_dispatch_stack() > 0 or torch._C._len_torch_function_stack() > 0
-            or torch.autograd.forward_ad._current_level >= 0 or torch.compiler.is_compiling() or torch.jit.is_tracing()
-            or torch._C._functorch.maybe_current_level() is not None
-            or bool(m._global_forward_hooks or m._global_forward_pre_hooks or m._global_backward_hooks or m._global_backward_pre_hooks))
+    gradients, a function transform, a hook on every module.  Some of these torch tells under private names only; where one
+    is gone, the individual operations run."""
+    try:
+        m, c = torch.nn.modules.module, torch._C
+        return (torch.is_autocast_enabled("cuda") or c._len_torch_dispatch_stack() > 0 or c._len_torch_function_stack() > 0
+                or torch.autograd.forward_ad._current_level >= 0 or torch.compiler.is_compiling() or torch.jit.is_tracing()
+                or c._functorch.maybe_current_level() is not None
+                or bool(m._global_forward_hooks or m._global_forward_pre_hooks or m._global_backward_hooks or m._global_backward_pre_hooks))
+    except AttributeError:
+        return True
+
+
+def plain_linear(m) -> bool:
+    """An ``nn.Linear`` with nothing attached to it: its output is ``F.linear`` of its weight and bias."""
+    if type(m) is not torch.nn.Linear:
+        return False
+    d = m.__dict__
+    return not (d.get("_forward_hooks", True) or d.get("_forward_pre_hooks", True) or d.get("_backward_hooks", True)
+                or d.get("_backward_pre_hooks", True) or "forward" in d)
 
 
 def linears_supported(x: Tensor, *linears) -> bool:
@@ -380,12 +393,10 @@ def linears_supported(x: Tensor, *linears) -> bool:
     if not (torch.is_grad_enabled() and type(x) is Tensor and x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and x.numel() > 0):
         return False
     for m in linears:
-        if type(m) is not torch.nn.Linear:
+        if not plain_linear(m):
             return False
-        d = m.__dict__
-        if d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"] or "forward" in d:
-            return False
-        w, b = d["_parameters"].get("weight"), d["_parameters"].get("bias")
+        p = m.__dict__["_parameters"]              # (a parametrised or deleted one is not in the table)
+        w, b = p.get("weight"), p.get("bias")
         if w is None or b is None or w.dtype != torch.bfloat16 or b.dtype != torch.bfloat16 or not (w.requires_grad and b.requires_grad):
             return False
         if w.device != x.device or m.out_features % 64 or type(w) is not torch.nn.Parameter or type(b) is not torch.nn.Parameter:

@@ -12,9 +12,9 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 from torch import Tensor
-from torch.nn.modules import module as _nn_module
 
 from flash_pop_b200 import _lib
+from flash_pop_b200.layer_ops import observed, plain_linear
 from flash_pop_b200.recurrent_state import RecurrentState
 from flash_pop_b200.xpos_emb import XPos
 
@@ -23,31 +23,16 @@ _BF, _F32 = torch.bfloat16, torch.float32
 _ACTS = {F.silu: _lib.ACT_SWISH, F.gelu: _lib.ACT_GELU, F.relu: _lib.ACT_RELU}
 
 
-def _global_hooks() -> bool:
-    m = _nn_module
-    return bool(m._global_forward_hooks or m._global_forward_pre_hooks or m._global_backward_hooks or m._global_backward_pre_hooks)
-
-
-def _watched() -> bool:
-    """Something that wants to see the individual operations."""
-    return (torch.is_grad_enabled() or torch.is_autocast_enabled("cuda") or torch._C._len_torch_dispatch_stack() > 0
-            or torch._C._len_torch_function_stack() > 0 or torch.autograd.forward_ad._current_level >= 0
-            or torch.compiler.is_compiling() or torch.jit.is_tracing() or _global_hooks())
-
-
 def _linear(m, n_out, n_in, device, out: list) -> bool:
-    if type(m) is not nn.Linear:
+    if not plain_linear(m):
         return False
-    d = m.__dict__
-    if d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"] or "forward" in d:
-        return False
-    p = d["_parameters"]
+    p = m.__dict__["_parameters"]
     address = _lib.native().address           # of a parameter that the kernels can read in place, or None
     w = address(p.get("weight"), _BF, 16, device, n_out, n_in)
     if w is None:
         return False
-    b = p.get("bias", d)                      # (a parametrised or deleted bias is not in the table at all)
-    if b is d:
+    b = p.get("bias", p)                      # (a parametrised or deleted bias is not in the table at all)
+    if b is p:
         return False
     b = 0 if b is None else address(b, _BF, 4, device, n_out, 0)
     if b is None:
@@ -120,7 +105,7 @@ def _layer(layer, first, shape, x_device, index, layer_cls, retention_cls):
 
 def decoder_token(net, x: Tensor, recurrent_state: Optional[RecurrentState], layer_cls, retention_cls):
     """``net.forward_recurrent(x, recurrent_state)`` through the fused launch, or None when the call is not one of theirs."""
-    if _watched() or type(x) is not Tensor or not x.is_cuda or x.dtype != _BF or x.dim() != 2 or not x.is_contiguous():
+    if torch.is_grad_enabled() or observed() or type(x) is not Tensor or not x.is_cuda or x.dtype != _BF or x.dim() != 2 or not x.is_contiguous():
         return None
     B, device = x.shape[0], x.device
     layers = list(net.layers)
