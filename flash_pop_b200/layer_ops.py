@@ -414,6 +414,13 @@ def _bias_grad(g: Tensor) -> Tensor:
     return g.sum(dim=tuple(range(g.dim() - 1)))
 
 
+def _wanted(ctx) -> Tuple[bool, ...]:
+    """Which of a Function's input gradients the running backward uses.  (`needs_input_grad` also names the weights when
+    autograd.grad asks for the gradient of the input alone, where the framework's own nodes leave their products out.)"""
+    fast = _lib.native().wanted(ctx)
+    return ctx.needs_input_grad if fast is None else fast
+
+
 def _rows2(t: Tensor) -> Tensor:
     return t.reshape(-1, t.size(-1))
 
@@ -431,15 +438,15 @@ class SharedInputLinears(torch.autograd.Function):
     @staticmethod
     def backward(ctx, *grads):
         x, *weights = ctx.saved_tensors
-        x2, dx, out = _rows2(x), None, []
+        x2, dx, out, need = _rows2(x), None, [], _wanted(ctx)
         for i, (g, w) in enumerate(zip(grads, weights)):
             if g is None:
                 out += (None, None)
                 continue
-            need_w, need_b = ctx.needs_input_grad[1 + 2 * i], ctx.needs_input_grad[2 + 2 * i]
+            need_w, need_b = need[1 + 2 * i], need[2 + 2 * i]
             g2 = _rows2(g)
             db = _bias_grad(g) if need_b else None         # (first: it binds the device to this thread, which cuBLAS wants done)
-            if ctx.needs_input_grad[0]:
+            if need[0]:
                 # (in place where no graph of this backward is wanted: out of place the sum is copied first)
                 dx = g2.mm(w) if dx is None else torch.addmm(dx, g2, w) if torch.is_grad_enabled() else dx.addmm_(g2, w)
             out += (g2.t().mm(x2) if need_w else None, db)
@@ -467,7 +474,7 @@ class SwishFeedForward(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, a, h, w1, w2, b1, b2 = ctx.saved_tensors
-        need = ctx.needs_input_grad
+        need = _wanted(ctx)
         if torch.is_grad_enabled():          # a graph of this backward is wanted: through the framework's own operations
             inputs = (x, w1, b1, w2, b2)
             y = torch.nn.functional.linear(torch.nn.functional.silu(torch.nn.functional.linear(x, w1, b1)), w2, b2)
@@ -476,6 +483,8 @@ class SwishFeedForward(torch.autograd.Function):
         dy2 = _rows2(dy)
         db2 = _bias_grad(dy) if need[4] else None      # (first: it binds the device to this thread, which cuBLAS wants done)
         dw2 = dy2.t().mm(_rows2(h)) if need[3] else None
+        if not any(need[:3]):
+            return None, None, None, dw2, db2
         dh = dy2.mm(w2).view(a.shape)
         fast = _lib.result(_lib.native().column_sums(dh, a))
         if fast is not None:

@@ -16,6 +16,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/DynamicTypes.h>
+#include <torch/csrc/autograd/python_function.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../include/flash_pop_b200.h"
@@ -494,6 +495,19 @@ PyObject* address(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+// wanted(ctx) -> per tensor input of the autograd Function whose backward runs, whether this backward uses its gradient:
+// an input that requires none, or that autograd.grad(..., inputs) leaves out, does not (needs_input_grad tells the first only)
+PyObject* wanted(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 1 || !THPFunction_Check(a[0])) Py_RETURN_NONE;
+  const auto node = reinterpret_cast<THPFunction*>(a[0])->cdata.lock();
+  if (!node) Py_RETURN_NONE;
+  const Py_ssize_t outputs = (Py_ssize_t)node->num_outputs();
+  PyObject* r = PyTuple_New(outputs);
+  if (!r) return nullptr;
+  for (Py_ssize_t i = 0; i < outputs; ++i) PyTuple_SET_ITEM(r, i, PyBool_FromLong(node->task_should_compute_output((size_t)i)));
+  return r;
+}
+
 // bind(addresses): the C ABI's entry points in the order of `Entry`
 PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != ENTRIES) { PyErr_SetString(PyExc_TypeError, "wrong number of entry points"); return nullptr; }
@@ -508,7 +522,7 @@ PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 #define FAST(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {FAST(step), FAST(forward), FAST(backward), FAST(suffix_forward), FAST(suffix_backward), FAST(rotary), FAST(gate_forward),
-                         FAST(gate_backward), FAST(norm_forward), FAST(norm_backward), FAST(column_sums), FAST(address), FAST(bind), {nullptr, nullptr, 0, nullptr}};
+                         FAST(gate_backward), FAST(norm_forward), FAST(norm_backward), FAST(column_sums), FAST(address), FAST(wanted), FAST(bind), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "fpb_fast_calls", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

@@ -4,7 +4,7 @@ import torch
 import torch.nn as nn
 from torch.utils.flop_counter import FlopCounterMode
 
-from flash_pop_b200 import layer_ops, token_stack
+from flash_pop_b200 import _lib, layer_ops, token_stack
 
 
 def test_nothing_is_watching():
@@ -62,3 +62,59 @@ def test_plain_linear():
     hooked[3].register_full_backward_pre_hook(lambda *a: None)
     hooked[4].forward = lambda t: t
     assert not any(layer_ops.plain_linear(m) for m in (Sub(2, 2), nn.Identity(), None, *hooked))
+
+
+def _grouped():
+    """The Functions of the training path and the modules they stand in for, on the CPU (fp32): (function, plain, leaves)."""
+    torch.manual_seed(0)
+    p = lambda *s: nn.Parameter(torch.randn(*s) * 0.1)
+    x, ws, bs = torch.randn(2, 9, 64, requires_grad=True), [p(64, 64) for _ in range(3)], [p(64) for _ in range(3)]
+    F = torch.nn.functional
+    yield (lambda h: sum(o.square().sum() for o in layer_ops.SharedInputLinears.apply(h, *(t for pair in zip(ws, bs) for t in pair))),
+           lambda h: sum(F.linear(h, w, b).square().sum() for w, b in zip(ws, bs)), x, [*ws, *bs])
+    w1, b1, w2, b2 = p(128, 64), p(128), p(64, 128), p(64)
+    yield (lambda h: layer_ops.SwishFeedForward.apply(h, w1, b1, w2, b2).square().sum(),
+           lambda h: F.linear(F.silu(F.linear(h, w1, b1)), w2, b2).square().sum(), x, [w1, b1, w2, b2])
+
+
+def _close(a, b):
+    # the same products added up in another order: a random walk over some 10^3 roundings of 2^-24, 2e-6 of the tensor's norm
+    assert float((a - b).norm()) <= 1e-5 * float(b.norm())
+
+
+@pytest.mark.parametrize("which", [0, 1])
+def test_only_the_gradients_asked_for_are_made(which):
+    """autograd.grad(y, x) and backward(inputs=...) cost no more products than through the modules, and every subset of
+    the gradients is right."""
+    _lib.build()
+    function, plain, x, params = list(_grouped())[which]
+
+    def grads(f, wanted):
+        h = x * 1
+        y = f(h)
+        with FlopCounterMode(display=False) as count:
+            got = torch.autograd.grad(y, [h if t is x else t for t in wanted])
+        return got, count.get_total_flops()
+
+    for wanted in ([x], [params[0]], params[-1:], params, [x, params[1]], [x, *params]):
+        got, flops = grads(function, wanted)
+        want, most = grads(plain, wanted)
+        assert flops <= most, (flops, most)
+        for a, b in zip(got, want):
+            _close(a, b)
+    for p in params:
+        p.grad = None
+    function(x).backward(inputs=[params[0]])
+    assert params[0].grad is not None and x.grad is None and all(p.grad is None for p in params[1:])
+    frozen = [p.requires_grad_(False) for p in params[:1]]
+    got, _ = grads(function, [x])
+    for a, b in zip(got, grads(plain, [x])[0]):
+        _close(a, b)
+    assert not any(p.requires_grad for p in frozen)
+    params[0].requires_grad_(True)
+    h = x * 1                                          # a graph of the backward: second derivatives, of a subset too
+    (g,) = torch.autograd.grad(function(h), [h], create_graph=True)
+    (g0,) = torch.autograd.grad(plain(h), [h], create_graph=True)
+    second = lambda t: torch.autograd.grad(t.square().sum(), [x, params[0]], retain_graph=True)
+    for a, b in zip(second(g), second(g0)):
+        _close(a, b)
