@@ -142,6 +142,16 @@ __global__ void __launch_bounds__(BCfg<DK, DV>::NTHREADS, 1) bwd_fused_kernel(co
   const float rs = rsqrtf((float)p.dk);
   const int NC = chunk_count(t_end - t0, p.block_size);
   auto bar = [&](int slot) { return sbase + G::OFF_BAR + slot * 8; };
+  // (Grouping of suffixes is compiled into the 64 x 64 kernel only - the shape suffixes come in; in the larger tiles its few
+  // extra live registers spill the state, which costs the long-sequence workloads far more than grouping gains.)
+  constexpr bool GROUPED = DK == 64 && DV == 64;
+  // (token, batch) coordinates in the tensor maps: grouped suffixes are batch entries of their own there, so that rows past
+  // a suffix's end read as zeros and are clipped on store
+  auto place = [&](int a) {
+    if (!GROUPED || p.sfx_G <= 1) return make_int2(a, b);
+    const int f = a / p.block_size;
+    return make_int2(a - f * p.block_size, f);
+  };
   auto stage_of = [&](int n) { return n % G::STAGES; };
   auto stage_ph = [&](int n) { return (uint32_t)((n / G::STAGES) & 1); };
   // tensor-memory addresses (lane offset in the upper half-word)
@@ -188,15 +198,16 @@ __global__ void __launch_bounds__(BCfg<DK, DV>::NTHREADS, 1) bwd_fused_kernel(co
         if (c == p.tune.withhold_chunk) { prev_chunk(ck, p.block_size); continue; }   // diagnostics: this chunk never arrives
         const uint32_t st = sbase + G::OFF_STAGE + s * G::STAGE_BYTES;
         mbar_arrive_expect_tx(bar(B_FULL + s), G::STAGE_BYTES);
+        const int2 at = place(ck.a);
 #pragma unroll
         for (int cb = 0; cb < DV / 64; ++cb) {      // dO first: it has to be scaled before anything can use it
-          tma_load_4d(st + G::OFF_DO + cb * 8192, &p.map_do, bar(B_FULL + s), vcol + cb * 64, ck.a, h, b);
-          tma_load_4d(st + G::OFF_V + cb * 8192, &p.map_v, bar(B_FULL + s), vcol + cb * 64, ck.a, h, b);
+          tma_load_4d(st + G::OFF_DO + cb * 8192, &p.map_do, bar(B_FULL + s), vcol + cb * 64, at.x, h, at.y);
+          tma_load_4d(st + G::OFF_V + cb * 8192, &p.map_v, bar(B_FULL + s), vcol + cb * 64, at.x, h, at.y);
         }
 #pragma unroll
         for (int cb = 0; cb < DK / 64; ++cb) {
-          tma_load_4d(st + G::OFF_Q + cb * 8192, &p.map_q, bar(B_FULL + s), cb * 64, ck.a, h, b);
-          tma_load_4d(st + G::OFF_K + cb * 8192, &p.map_k, bar(B_FULL + s), cb * 64, ck.a, h, b);
+          tma_load_4d(st + G::OFF_Q + cb * 8192, &p.map_q, bar(B_FULL + s), cb * 64, at.x, h, at.y);
+          tma_load_4d(st + G::OFF_K + cb * 8192, &p.map_k, bar(B_FULL + s), cb * 64, at.x, h, at.y);
         }
         ++issued;
         prev_chunk(ck, p.block_size);
@@ -394,19 +405,21 @@ __global__ void __launch_bounds__(BCfg<DK, DV>::NTHREADS, 1) bwd_fused_kernel(co
       const float z_lo = exp2f((float)(ck.L - 1 - r_lo) * lg) * rs, z_hi = exp2f((float)(ck.L - 9 - r_lo) * lg) * rs;
       acc_to_staging(tm_accv, sm + G::OFF_OUTV, DV, z_lo, z_hi, false);
       acc_to_staging(tm_acck, sm + G::OFF_OUTK, DK, z_lo, z_hi, true);
-      const bool whole_box = ck.L == C || ck.a + ck.L >= p.T;
+      // rows beyond L are past the end of the sequence, or of the suffix: TMA clips them
+      const bool whole_box = ck.L == C || ck.a + ck.L >= p.T || (GROUPED && p.sfx_G > 1);
       if (whole_box) fence_async_smem();
       named_bar_sync(2, N_SCORE);
       if (whole_box) {
         if (t == 0) {
+          const int2 at = place(ck.a);
 #pragma unroll
-          for (int cb = 0; cb < DV / 64; ++cb) tma_store_4d(&p.map_dv, sbase + G::OFF_OUTV + cb * 8192, vcol + cb * 64, ck.a, h, b);
+          for (int cb = 0; cb < DV / 64; ++cb) tma_store_4d(&p.map_dv, sbase + G::OFF_OUTV + cb * 8192, vcol + cb * 64, at.x, h, at.y);
           if (p.dk_add) {
 #pragma unroll
-            for (int cb = 0; cb < DK / 64; ++cb) tma_reduce_add_4d(&p.map_dk, sbase + G::OFF_OUTK + cb * 8192, cb * 64, ck.a, h, b);
+            for (int cb = 0; cb < DK / 64; ++cb) tma_reduce_add_4d(&p.map_dk, sbase + G::OFF_OUTK + cb * 8192, cb * 64, at.x, h, at.y);
           } else {
 #pragma unroll
-            for (int cb = 0; cb < DK / 64; ++cb) tma_store_4d(&p.map_dk, sbase + G::OFF_OUTK + cb * 8192, cb * 64, ck.a, h, b);
+            for (int cb = 0; cb < DK / 64; ++cb) tma_store_4d(&p.map_dk, sbase + G::OFF_OUTK + cb * 8192, cb * 64, at.x, h, at.y);
           }
           tma_store_commit();
         }
@@ -466,9 +479,6 @@ __global__ void __launch_bounds__(BCfg<DK, DV>::NTHREADS, 1) bwd_fused_kernel(co
     auto at = [&](const void* base, int64_t elems) { return (void*)((const char*)base + elems * esz); };
     // suffix calls: suffix f of the call is suffix f % M of row f / M; the walk goes through its piece's suffixes from the
     // last to the first, and what it carries when it leaves one is the gradient of the state that suffix started from
-    // (Grouping is compiled into the 64 x 64 kernel only - the shape suffixes come in; in the larger tiles its few
-    // extra live registers spill the state, which costs the long-sequence workloads far more than grouping gains.)
-    constexpr bool GROUPED = DK == 64 && DV == 64;
     const int sfx_g = GROUPED ? p.sfx_G : 1;
     auto sfx_grad = [&](int f) -> void* {
       const int row = f / p.sfx_M, m = f % p.sfx_M;
@@ -798,12 +808,12 @@ int launch_bwd_fused(const UmmaBwdArgs& a, cudaStream_t stream, int* n_launched)
       return r;
     *n_launched += 2;
   }
-  if ((r = make_seq_map(&p.map_q, q, B, T, H, a.dk, C)) != FPB_OK) return r;
-  if ((r = make_seq_map(&p.map_k, k, B, T, H, a.dk, C)) != FPB_OK) return r;
-  if ((r = make_seq_map(&p.map_v, v, B, T, H, a.dv, C)) != FPB_OK) return r;
-  if ((r = make_seq_map(&p.map_do, dO, B, T, H, a.dv, C)) != FPB_OK) return r;
-  if ((r = make_seq_map(&p.map_dk, dK, B, T, H, a.dk, C)) != FPB_OK) return r;
-  if ((r = make_seq_map(&p.map_dv, dV, B, T, H, a.dv, C)) != FPB_OK) return r;
+  if ((r = make_seq_map(&p.map_q, q, a.B, a.T, H, a.dk, C)) != FPB_OK) return r;
+  if ((r = make_seq_map(&p.map_k, k, a.B, a.T, H, a.dk, C)) != FPB_OK) return r;
+  if ((r = make_seq_map(&p.map_v, v, a.B, a.T, H, a.dv, C)) != FPB_OK) return r;
+  if ((r = make_seq_map(&p.map_do, dO, a.B, a.T, H, a.dv, C)) != FPB_OK) return r;
+  if ((r = make_seq_map(&p.map_dk, dK, a.B, a.T, H, a.dk, C)) != FPB_OK) return r;
+  if ((r = make_seq_map(&p.map_dv, dV, a.B, a.T, H, a.dv, C)) != FPB_OK) return r;
   if (a.dk == 64 && a.dv == 64 && !a.state_f32 && a.d_block_states && a.n_blocks > 0) {
     // (B, N, H, dk, dv) contiguous as a 4-D tensor of 64-wide rows: dk rows per (block, head), N * H of those per batch row
     const SeqView bg{const_cast<void*>(a.d_block_states), (int64_t)a.n_blocks * H * a.dk * a.dv, (int64_t)a.dv, (int64_t)a.dk * a.dv};
