@@ -207,6 +207,7 @@ _DIAG_SIGNATURES = {
     "fpb_debug_col_split": [ctypes.c_int],
     "fpb_debug_deep": [ctypes.c_int],
     "fpb_debug_ablate": [ctypes.c_int],
+    "fpb_debug_refuse_launch": [ctypes.c_int],
     "fpb_debug_tuning": [ctypes.c_longlong, ctypes.c_int, ctypes.c_int, ctypes.c_int],
 }
 

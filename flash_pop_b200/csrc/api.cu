@@ -136,6 +136,13 @@ int finish_launches(int n, int path) {
   return FPB_OK;
 }
 
+// The status of a launcher.  A failed launch's CUDA error is kept for fpb_last_cuda_error and taken off the thread: left
+// pending, the next call would find it and report it as its own.
+int launcher_status(int r) {
+  if (r == FPB_ERR_LAUNCH) tl_last_cuda_error = (int)cudaGetLastError();
+  return r;
+}
+
 void fill_common(WalkParams& p, const Call& c, int dir, const SuffixStates& sfx) {
   std::memset(&p, 0, sizeof(p));
   p.T = c.T; p.H = c.H; p.dk = c.dk; p.dv = c.dv; p.dir = dir;
@@ -170,7 +177,7 @@ int forward(const Call& c, int64_t batch, SeqView q, SeqView k, SeqView v, State
     int n_launched = 0;
     const int r = launch_umma_fwd(a, stream, &n_launched);
     if (r == FPB_OK) return finish_launches(n_launched, FPB_PATH_TCGEN05);
-    if (r != FPB_UMMA_NOT_APPLICABLE) return r;
+    if (r != FPB_UMMA_NOT_APPLICABLE) return launcher_status(r);
   }
   if (c.dtype == FPB_F32 && !block_states && sfx.M == 0) {
     ChunkArgs a = chunk_args(c, batch, q, k, v, s0);
@@ -178,7 +185,7 @@ int forward(const Call& c, int64_t batch, SeqView q, SeqView k, SeqView v, State
     int n_launched = 0;
     const int r = launch_chunk_fwd(a, stream, &n_launched);
     if (r == FPB_OK) return finish_launches(n_launched, FPB_PATH_SIMT);
-    if (r != FPB_CHUNK_NOT_APPLICABLE) { tl_last_cuda_error = (int)cudaGetLastError(); return r; }
+    if (r != FPB_CHUNK_NOT_APPLICABLE) return launcher_status(r);
   }
   WalkParams p;
   fill_common(p, c, +1, sfx);
@@ -207,7 +214,7 @@ int backward(const Call& c, int64_t batch, SeqView q, SeqView k, SeqView v, Stat
     int n_launched = 0;
     const int r = launch_umma_bwd(a, stream, &n_launched);
     if (r == FPB_OK) return finish_launches(n_launched, FPB_PATH_TCGEN05);
-    if (r != FPB_UMMA_NOT_APPLICABLE) return r;
+    if (r != FPB_UMMA_NOT_APPLICABLE) return launcher_status(r);
   }
   if (c.dtype == FPB_F32 && c.block_size == 0 && sfx_in.M == 0) {
     ChunkArgs a = chunk_args(c, batch, q, k, v, s0);
@@ -215,7 +222,7 @@ int backward(const Call& c, int64_t batch, SeqView q, SeqView k, SeqView v, Stat
     int n_launched = 0;
     const int r = launch_chunk_bwd(a, (c.flags & FPB_FLAG_SKIP_DQ) != 0, (c.flags & FPB_FLAG_SKIP_DKDV) != 0, stream, &n_launched);
     if (r == FPB_OK) return finish_launches(n_launched, FPB_PATH_SIMT);
-    if (r != FPB_CHUNK_NOT_APPLICABLE) { tl_last_cuda_error = (int)cudaGetLastError(); return r; }
+    if (r != FPB_CHUNK_NOT_APPLICABLE) return launcher_status(r);
   }
   WalkParams p;
   int r, n = 0;

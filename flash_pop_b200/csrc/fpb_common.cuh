@@ -132,6 +132,10 @@ int sm_count();              // of the current device
 int launch_segment_combine(float* seg, Segments sg, int B, int T, int H, int dk, int dv, const float* gamma, bool reverse,
                            StateView start, bool state_f32, cudaStream_t stream);
 
+#ifdef FPB_DIAGNOSTICS
+bool launch_refused();       // diagnostics: whether the runtime is to refuse this launch (fpb_debug_refuse_launch)
+#endif
+
 // Launch `kernel`; `chained`: it may start before the launch ahead of it has ended (programmatic dependent launch) and
 // waits inside, with griddepcontrol.wait, where it needs that launch's results.
 template <typename P>
@@ -142,6 +146,9 @@ cudaError_t launch_kernel(void (*kernel)(P), dim3 grid, int threads, size_t smem
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr; cfg.numAttrs = chained ? 1 : 0;
+#ifdef FPB_DIAGNOSTICS
+  if (launch_refused()) cfg.blockDim = dim3(0);
+#endif
   return cudaLaunchKernelEx(&cfg, kernel, p);
 }
 

@@ -1183,6 +1183,7 @@ FPB_KNOB g_col_split = 1;            // 1: dv = 256 gradient walks cut dv into 1
 #ifdef FPB_DIAGNOSTICS
 long long* g_trace = nullptr;        // set by fpb_debug_trace
 WalkTuning g_tuning{kWaitCycles, 200, 1, -1, 0};
+int g_refuse_launch = -1;            // launches until the one the runtime is to refuse (-1: none)
 #else
 constexpr long long* g_trace = nullptr;
 constexpr WalkTuning g_tuning{kWaitCycles, 200, 1, -1, 0};
@@ -1384,7 +1385,10 @@ int choose_suffix_group(int suffixes, long long units, int ctas_per_sm) {
 }
 
 #ifdef FPB_DIAGNOSTICS
+bool launch_refused() { return g_refuse_launch >= 0 && g_refuse_launch-- == 0; }
 // Hooks of the diagnostics build (not part of the public header).
+// Give the n-th launch from now on (0: the next) a block of no threads, which the runtime refuses on the host; -1: none.
+extern "C" void fpb_debug_refuse_launch(int n) { g_refuse_launch = n; }
 // Install a device buffer of 64*16 int64 that the next launches fill with clock64() stamps of their first CTA; null removes it.
 extern "C" void fpb_debug_trace(void* device_buffer) { g_trace = (long long*)device_buffer; }
 // Choose between the 128x128 state tiles (1, default) and the 64-wide ones (0).
