@@ -18,6 +18,8 @@
 // Bound by the FMA pipe and the shared-memory loads that feed it (16 FMAs per 16-byte load and thread at most); the chunk
 // is as short as it is because the work inside a chunk grows with its length and the number of CTAs falls.
 // Terms that the causal mask leaves out are never multiplied: an infinity in a later token must not reach an earlier one.
+// Nor is padding - tokens past the end of a ragged chunk, channels past the head dimension: 0 x infinity would turn a
+// token's own infinite gradient into NaN.
 #include <atomic>
 
 #include "fpb_common.cuh"
@@ -76,7 +78,7 @@ template <int DK, int DV> __device__ __forceinline__ void store_state(const floa
 // S <- decay S + sum over the chunk's n tokens of w_j A_j (x) B_j, w_j = pw[first + step * j]; a thread holds a
 // (DK/16) x (DV/16) block of S, rows side by side, columns in pieces of four
 template <int DK, int DV> __device__ __forceinline__ void update_state(float* S, const float* A, const float* B, const float* pw, int n,
-                                                                       int first, int step, float decay) {
+                                                                       int first, int step, float decay, int dk, int dv) {
   constexpr int TR = DK / 16, TC = DV / 16, CV = TC < 4 ? TC : 4, NC = TC / CV;
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
   float acc[TR][TC];
@@ -104,8 +106,9 @@ template <int DK, int DV> __device__ __forceinline__ void update_state(float* S,
   for (int r = 0; r < TR; ++r)
 #pragma unroll
     for (int c = 0; c < TC; ++c) {
-      float& x = s0[r * (DV + 4) + (c / CV) * (DV / NC) + c % CV];
-      x = fmaf(decay, x, acc[r][c]);
+      const int col = (c / CV) * (DV / NC) + c % CV;
+      float& x = s0[r * (DV + 4) + col];
+      if (ty * TR + r < dk && tx * CV + col < dv) x = fmaf(decay, x, acc[r][c]);
     }
 }
 
@@ -148,12 +151,13 @@ template <int R> __device__ __forceinline__ void add_to(float (&acc)[R][4], cons
 #pragma unroll
     for (int c = 0; c < 4; ++c) acc[r][c] += sum[r][c];
 }
-// acc += A[row] M  for the [K][N] matrix M (pitch N + 4)
-template <int K, int N> __device__ __forceinline__ void times(float (&acc)[N / 32][4], const float* A, const float* M, const Own<N>& own) {
-  for (int k0 = 0; k0 < K; k0 += 32) {
+// acc += A[row] M  for the [K][N] matrix M (pitch N + 4), of which the first `real` (a multiple of 4) rows count
+template <int K, int N> __device__ __forceinline__ void times(float (&acc)[N / 32][4], const float* A, const float* M, const Own<N>& own, int real) {
+  for (int k0 = 0; k0 < real; k0 += 32) {
     float sum[N / 32][4] = {};
+    const int k1 = min(k0 + 32, real);
 #pragma unroll 2
-    for (int k = k0; k < k0 + 32; k += 4) {
+    for (int k = k0; k < k1; k += 4) {
       float4 m[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) m[i] = *reinterpret_cast<const float4*>(M + (k + i) * (N + 4) + own.col);
@@ -171,12 +175,13 @@ template <int K, int N> __device__ __forceinline__ void times(float (&acc)[N / 3
     add_to<N / 32>(acc, sum);
   }
 }
-// acc += A[row] M^T for the [N][K] matrix M (pitch K + 4), columns N/4 apart
-template <int K, int N> __device__ __forceinline__ void times_t(float (&acc)[N / 32][4], const float* A, const float* M, const Own<N>& own) {
-  for (int k0 = 0; k0 < K; k0 += 32) {
+// acc += A[row] M^T for the [N][K] matrix M (pitch K + 4, `real` columns of it), columns N/4 apart
+template <int K, int N> __device__ __forceinline__ void times_t(float (&acc)[N / 32][4], const float* A, const float* M, const Own<N>& own, int real) {
+  for (int k0 = 0; k0 < real; k0 += 32) {
     float sum[N / 32][4] = {};
+    const int k1 = min(k0 + 32, real);
 #pragma unroll 2
-    for (int k = k0; k < k0 + 32; k += 4) {
+    for (int k = k0; k < k1; k += 4) {
       float4 m[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) m[i] = *reinterpret_cast<const float4*>(M + (own.col + i * (N / 4)) * (K + 4) + k);
@@ -190,14 +195,14 @@ template <int K, int N> __device__ __forceinline__ void times_t(float (&acc)[N /
     add_to<N / 32>(acc, sum);
   }
 }
-// acc += P[row] M over the causal side of the 32 x 32 tile P (y <= row, or y >= row with UP), M [32][N]
+// acc += P[row] M over the causal side of the 32 x 32 tile P (y <= row, or row <= y < n with UP), M [32][N]
 template <int N, bool STRIDED, bool UP> __device__ __forceinline__ void times_scores(float (&acc)[N / 32][4], const float* P, const float* M,
-                                                                                    const Own<N>& own) {
+                                                                                    const Own<N>& own, int n) {
   constexpr int R = N / 32;
   float sum[R][4] = {};
-  const int lo = UP ? own.row & ~3 : 0, hi = UP ? L32 : (own.row + R + 3) & ~3;
+  const int lo = UP ? own.row & ~3 : 0, hi = UP ? (n + 3) & ~3 : (own.row + R + 3) & ~3;
   for (int k = lo; k < hi; k += 4) {
-    const bool whole = UP ? k >= own.row + R - 1 : k + 3 <= own.row;
+    const bool whole = UP ? k >= own.row + R - 1 && k + 3 < n : k + 3 <= own.row;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       float4 m;
@@ -207,7 +212,7 @@ template <int N, bool STRIDED, bool UP> __device__ __forceinline__ void times_sc
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const int row = own.row + r;
-        if (whole || (UP ? k + i >= row : k + i <= row)) {
+        if (whole || (UP ? k + i >= row && k + i < n : k + i <= row)) {
           const float e = P[row * PP + k + i];
           sum[r][0] = fmaf(e, m.x, sum[r][0]); sum[r][1] = fmaf(e, m.y, sum[r][1]);
           sum[r][2] = fmaf(e, m.z, sum[r][2]); sum[r][3] = fmaf(e, m.w, sum[r][3]);
@@ -269,7 +274,7 @@ __global__ void __launch_bounds__(THREADS) chunk_segments_kernel(const __grid_co
     load_tile<DK>(A, rev ? p.q : p.k, b, h, a, n, p.dk, rev ? 1.0f : rs);
     load_tile<DV>(B, rev ? p.dO : p.v, b, h, a, n, p.dv, 1.0f);
     __syncthreads();
-    update_state<DK, DV>(S, A, B, pw, n, rev ? 1 : n - 1, rev ? 1 : -1, pw[n]);
+    update_state<DK, DV>(S, A, B, pw, n, rev ? 1 : n - 1, rev ? 1 : -1, pw[n], p.dk, p.dv);
     __syncthreads();
   }
   grid_wait();                                     // (the first of the chain: nothing to wait for)
@@ -341,12 +346,12 @@ __global__ void __launch_bounds__(THREADS) chunk_fwd_kernel(const __grid_constan
     __syncthreads();
     scores<DK, false>(P, Q, K, pw);
     float acc[DV / 32][4] = {};
-    times<DK, DV>(acc, Q, S, own);
+    times<DK, DV>(acc, Q, S, own, p.dk);
     scale_rows<DV>(acc, own, pw, 1, 1, n);
     __syncthreads();
-    times_scores<DV, false, false>(acc, P, V, own);
+    times_scores<DV, false, false>(acc, P, V, own, n);
     store_rows<DV, false>(acc, own, p.o, b, h, a, n, p.dv, 1.0f);
-    if (a + L32 < t1 || ends) update_state<DK, DV>(S, K, V, pw, n, n - 1, -1, pw[n]);   // (S was last read before the barrier)
+    if (a + L32 < t1 || ends) update_state<DK, DV>(S, K, V, pw, n, n - 1, -1, pw[n], p.dk, p.dv);   // (S was last read before the barrier)
     __syncthreads();
   }
   if (ends) store_state<DK, DV>(S, (float*)p.s_out.data + b * p.s_out.sb + h * p.s_out.sh, p.dk, p.dv);
@@ -380,27 +385,27 @@ __global__ void __launch_bounds__(THREADS) chunk_bwd_kernel(const __grid_constan
     if (!rev) {
       scores<DV, false>(P2, D, V, pw);
       float acc[DK / 32][4] = {};
-      times_t<DV, DK>(acc, D, S, own_k);
+      times_t<DV, DK>(acc, D, S, own_k, p.dv);
       scale_rows<DK>(acc, own_k, pw, 1, 1, n);
       __syncthreads();
-      times_scores<DK, true, false>(acc, P2, K, own_k);
+      times_scores<DK, true, false>(acc, P2, K, own_k, n);
       store_rows<DK, true>(acc, own_k, p.dQ, b, h, a, n, p.dk, 1.0f);
-      if (c + 1 < chunks) update_state<DK, DV>(S, K, V, pw, n, n - 1, -1, pw[n]);
+      if (c + 1 < chunks) update_state<DK, DV>(S, K, V, pw, n, n - 1, -1, pw[n], p.dk, p.dv);
     } else {
       scores<DK, true>(P1, K, Q, pw);              // (K carries rs)
       scores<DV, true>(P2, V, D, pw);
       float av[DV / 32][4] = {};
-      times<DK, DV>(av, K, S, own_v);
+      times<DK, DV>(av, K, S, own_v, p.dk);
       scale_rows<DV>(av, own_v, pw, n - 1, -1, n);
       float ak[DK / 32][4] = {};
-      times_t<DV, DK>(ak, V, S, own_k);
+      times_t<DV, DK>(ak, V, S, own_k, p.dv);
       scale_rows<DK>(ak, own_k, pw, n - 1, -1, n);
       __syncthreads();
-      times_scores<DV, false, true>(av, P1, D, own_v);
+      times_scores<DV, false, true>(av, P1, D, own_v, n);
       store_rows<DV, false>(av, own_v, p.dV, b, h, a, n, p.dv, 1.0f);
-      times_scores<DK, true, true>(ak, P2, Q, own_k);
+      times_scores<DK, true, true>(ak, P2, Q, own_k, n);
       store_rows<DK, true>(ak, own_k, p.dK, b, h, a, n, p.dk, rs);
-      if (c + 1 < chunks || (seg == 0 && p.g_out.data)) update_state<DK, DV>(S, Q, D, pw, n, 1, 1, pw[n]);
+      if (c + 1 < chunks || (seg == 0 && p.g_out.data)) update_state<DK, DV>(S, Q, D, pw, n, 1, 1, pw[n], p.dk, p.dv);
     }
     __syncthreads();
   }

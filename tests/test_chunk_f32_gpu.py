@@ -116,3 +116,28 @@ def test_scratch_limits_change_the_split_only():
         _lib.check(_lib.lib().fpb_retention_fwd_static(_lib.dims(q, d, decays), _lib.seq(q), _lib.seq(k), _lib.seq(v), _lib.state(s),
                                                        _lib.seq(o2), _lib.state(None), _lib.stream_ptr(q.device)))
         assert _rel(o2, ref) < REL
+
+
+@pytest.mark.parametrize("T,dk,dv", [(70, 32, 64), (70, 36, 20), (33, 128, 100), (300, 20, 128)])
+def test_padding_meets_no_infinity(T, dk, dv):
+    """Everything positive and one infinity: every sum is finite or +inf, with no 0 x inf unless padding is multiplied.
+    The token walk (which unaligned tensors take) pads nothing and says which elements are which."""
+    import flash_pop_b200 as fp
+    B, H = 1, 2
+    decays = orc.head_decays(H, (5, 12))
+    q, k, v, s, dO, dS = (t.abs().cuda() + 0.01 for t in _inputs(13, B, T, H, dk, dv))
+
+    def unaligned(t):
+        return torch.empty(t.numel() + 1, device="cuda")[1:].view(t.shape).copy_(t)
+
+    def run(form):
+        x = [form(t).requires_grad_(True) for t in (q2, k2, v2, s)]
+        o, s_out = fp.fused_chunk_retention(*x, decays)
+        return [o, s_out, *torch.autograd.grad((o, s_out), x, (form(dO), dS))]
+
+    for token in (T - 1, T - 3, T // 2):
+        for which in range(3):
+            q2, k2, v2 = (t.clone() for t in (q, k, v))
+            (q2, k2, v2)[which][0, token, 1, 3] = float("inf")
+            for a, b in zip(run(lambda t: t.clone()), run(unaligned)):
+                assert not torch.isnan(b).any() and torch.equal(torch.isinf(a), torch.isinf(b)) and not torch.isnan(a).any()
