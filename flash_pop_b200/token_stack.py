@@ -23,25 +23,29 @@ _BF, _F32 = torch.bfloat16, torch.float32
 _ACTS = {F.silu: _lib.ACT_SWISH, F.gelu: _lib.ACT_GELU, F.relu: _lib.ACT_RELU}
 
 
-def _linear(m, n_out, n_in, device, out: list) -> bool:
+# `kept` holds every tensor whose address goes into the launch until it is made: between the two another thread may replace
+# a parameter or grow a table, and what it lets go would be handed out again.
+def _linear(m, n_out, n_in, device, out: list, kept: list) -> bool:
     if not plain_linear(m):
         return False
     p = m.__dict__["_parameters"]
     address = _lib.native().address           # of a parameter that the kernels can read in place, or None
-    w = address(p.get("weight"), _BF, 16, device, n_out, n_in)
+    weight = p.get("weight")
+    w = address(weight, _BF, 16, device, n_out, n_in)
     if w is None:
         return False
-    b = p.get("bias", p)                      # (a parametrised or deleted bias is not in the table at all)
-    if b is p:
+    bias = p.get("bias", p)                   # (a parametrised or deleted bias is not in the table at all)
+    if bias is p:
         return False
-    b = 0 if b is None else address(b, _BF, 4, device, n_out, 0)
+    b = 0 if bias is None else address(bias, _BF, 4, device, n_out, 0)
     if b is None:
         return False
     out += (w, b)
+    kept += (weight, bias)
     return True
 
 
-def _norm(m, width, device, out: list) -> bool:
+def _norm(m, width, device, out: list, kept: list) -> bool:
     if type(m) is not nn.LayerNorm or m.normalized_shape != (width,) or "forward" in m.__dict__:
         return False
     d = m.__dict__["_parameters"]
@@ -49,14 +53,15 @@ def _norm(m, width, device, out: list) -> bool:
         t = d.get(name, m)
         if t is m:
             return False
-        t = 0 if t is None else _lib.native().address(t, _F32, 16, device, width, 0)
-        if t is None:
+        at = 0 if t is None else _lib.native().address(t, _F32, 16, device, width, 0)
+        if at is None:
             return False
-        out.append(t)
+        out.append(at)
+        kept.append(t)
     return True
 
 
-def _layer(layer, first, shape, x_device, index, layer_cls, retention_cls):
+def _layer(layer, first, shape, x_device, index, layer_cls, retention_cls, kept: list):
     """(pointers, phasor address, tail of the layer's record) of a layer the kernels can run as it stands, else None."""
     H, dk, dv, ffn = shape
     width, device = H * dv, x_device.index
@@ -85,11 +90,11 @@ def _layer(layer, first, shape, x_device, index, layer_cls, retention_cls):
     rm = rown["_modules"]
     ptrs: list = []
     n1, n2 = mods["norm1"], mods["norm2"]
-    if not (_norm(n1, width, device, ptrs) and _norm(n2, width, device, ptrs)
-            and _linear(rm["q_proj"], H * dk, width, device, ptrs) and _linear(rm["k_proj"], H * dk, width, device, ptrs)
-            and _linear(rm["v_proj"], width, width, device, ptrs) and _linear(rm["g_proj"], width, width, device, ptrs)
-            and _linear(rm["out_proj"], width, width, device, ptrs) and _linear(mods["linear1"], ffn, width, device, ptrs)
-            and _linear(mods["linear2"], width, ffn, device, ptrs)):
+    if not (_norm(n1, width, device, ptrs, kept) and _norm(n2, width, device, ptrs, kept)
+            and _linear(rm["q_proj"], H * dk, width, device, ptrs, kept) and _linear(rm["k_proj"], H * dk, width, device, ptrs, kept)
+            and _linear(rm["v_proj"], width, width, device, ptrs, kept) and _linear(rm["g_proj"], width, width, device, ptrs, kept)
+            and _linear(rm["out_proj"], width, width, device, ptrs, kept) and _linear(mods["linear1"], ffn, width, device, ptrs, kept)
+            and _linear(mods["linear2"], width, ffn, device, ptrs, kept)):
         return None
     if ret.relative_position:
         xpos = ret.xpos_embedder
@@ -98,6 +103,7 @@ def _layer(layer, first, shape, x_device, index, layer_cls, retention_cls):
         xpos._move(x_device)
         row = xpos._rotation(1, index)
         ptrs.append(row.data_ptr())
+        kept.append(row)
     else:
         ptrs.append(0)
     return ptrs, (act_gate, act_ffn, n1.eps, n2.eps, rm["group_norm"].eps)
@@ -161,8 +167,9 @@ def decoder_token(net, x: Tensor, recurrent_state: Optional[RecurrentState], lay
     table = bytearray(n * size)
     out = torch.empty((n, B, H, dk, dv), device=device, dtype=out_dtype)
     out_base, out_step = out.data_ptr(), out.stride(0) * out.element_size()
+    kept = [states]
     for i, layer in enumerate(layers):
-        got = _layer(layer, first, (H, dk, dv, ffn), device, index, layer_cls, retention_cls)
+        got = _layer(layer, first, (H, dk, dv, ffn), device, index, layer_cls, retention_cls, kept)
         if got is None:
             return None
         record.pack_into(table, i * size, *got[0], addresses[i], sb, sh, out_base + i * out_step, out.stride(1), out.stride(2), *got[1])

@@ -131,3 +131,38 @@ def test_calls_that_keep_the_layer_by_layer_path():
         dropping.train()
         assert not taken(dropping)
     assert not taken(_net(1, 4, 64, 64, 256))        # gradients on
+
+
+def test_what_the_launch_reads_is_alive_until_it_is_made(monkeypatch):
+    """Another thread may replace a parameter or grow the rotation table while the addresses are collected."""
+    import weakref
+    import flash_pop_b200 as fp
+    from flash_pop_b200 import _lib
+    net = _net(2, 4, 64, 64, 256)
+    x = torch.randn(3, 256, device="cuda").to(BF)
+    real, refs, alive = _lib.lib(), [], []
+    xpos, q_proj = net.xpos_embedder, net.layers[0].retention.q_proj
+    table_row = xpos._rotation
+
+    def rotation(length, index):
+        row = table_row(length, index).clone()                  # (as a table that is replaced at once)
+        if refs:
+            refs.append(weakref.ref(q_proj.weight))
+            q_proj.weight = torch.nn.Parameter(q_proj.weight.clone(), requires_grad=False)
+        refs.append(weakref.ref(row))
+        return row
+
+    class Lib:
+        def __getattr__(self, name):
+            return getattr(real, name)
+
+        def fpb_decoder_token(self, *args):
+            alive.extend(r() is not None for r in refs)
+            return real.fpb_decoder_token(*args)
+
+    with torch.no_grad():
+        want, _ = net.forward_recurrent(x, fp.RecurrentState(None, 5))
+        monkeypatch.setattr(xpos, "_rotation", rotation)
+        monkeypatch.setattr(_lib, "lib", lambda handle=Lib(): handle)
+        got, _ = net.forward_recurrent(x, fp.RecurrentState(None, 5))
+    assert alive == [True] * 3 and torch.equal(got, want)
