@@ -318,9 +318,10 @@ class RetNetDecoder(nn.Module):
         return x, RecurrentState(torch.stack(states), rs.index + advance)
 
     def forward_recurrent(self, x: Tensor, recurrent_state: RecurrentState = None) -> Tuple[Tensor, RecurrentState]:
-        fused = decoder_token(self, x, recurrent_state, RetNetDecoderLayer, MultiScaleRetention)
-        if fused is not None:
-            return fused
+        if type(self)._walk_layers is RetNetDecoder._walk_layers and "_walk_layers" not in self.__dict__:
+            fused = decoder_token(self, x, recurrent_state, RetNetDecoderLayer, MultiScaleRetention)
+            if fused is not None:
+                return fused
         return self._walk_layers(x, recurrent_state, lambda layer, h, idx, st: layer.forward_recurrent(h, idx, st), 1)
 
     def forward_chunkwise(self, x: Tensor, recurrent_state: RecurrentState = None) -> Tuple[Tensor, RecurrentState]:

@@ -166,3 +166,27 @@ def test_what_the_launch_reads_is_alive_until_it_is_made(monkeypatch):
         monkeypatch.setattr(_lib, "lib", lambda handle=Lib(): handle)
         got, _ = net.forward_recurrent(x, fp.RecurrentState(None, 5))
     assert alive == [True] * 3 and torch.equal(got, want)
+
+
+def test_an_overridden_walk_over_the_layers_is_taken():
+    """A decoder class, or one decoder, that walks its layers in its own way does so for a token as for a chunk."""
+    import flash_pop_b200 as fp
+    net = _net(2, 4, 64, 64, 256)
+    x = torch.randn(3, 256, device="cuda").to(BF)
+    walked = []
+
+    class Own(fp.RetNetDecoder):
+        def _walk_layers(self, *args):
+            walked.append(self)
+            return super()._walk_layers(*args)
+
+    with torch.no_grad():
+        net.forward_recurrent(x)
+        net.__class__ = Own
+        net.forward_recurrent(x)
+        assert len(walked) == 1
+        net.__class__ = fp.RetNetDecoder
+        plain = net._walk_layers
+        net._walk_layers = lambda *args: walked.append(net) or plain(*args)
+        net.forward_recurrent(x)
+        assert len(walked) == 2
