@@ -37,6 +37,32 @@ def _layouts(t):
     return {"plain": t, "packed": packed, "turned": turned, "odd": odd, "expanded": t[:1].expand_as(t), "inner": t.transpose(-1, -2).contiguous().transpose(-1, -2)}
 
 
+class _Recorder:
+    """The extension, with a note of which of its functions took the call they were given."""
+
+    def __init__(self, native):
+        self.native, self.taken = native, {}
+
+    def __getattr__(self, name):
+        def call(*args):
+            got = getattr(self.native, name)(*args)
+            self.taken.setdefault(name, []).append(got is not None)
+            return got
+        return call
+
+
+@contextlib.contextmanager
+def recorded():
+    from flash_pop_b200 import _lib
+    kept = _lib.native
+    recorder = _Recorder(kept())
+    _lib.native = lambda: recorder
+    try:
+        yield recorder.taken
+    finally:
+        _lib.native = kept
+
+
 def _both(f):
     """f() on the native path and on the Python path: results, or the type and text of what was raised."""
     def attempt():
@@ -134,3 +160,76 @@ def test_layer_passes():
 
             for f in (rotary, gate, norm):
                 _both(f)
+
+
+@pytest.mark.parametrize("layout", ["plain", "packed", "turned", "odd", "expanded", "inner"])
+@pytest.mark.parametrize("dtype,state", [(BF, BF), (BF, F32), (BF, None), (F32, F32), (F32, None)])
+def test_the_extension_takes_the_ordinary_call(layout, dtype, state):
+    """Which calls go through the extension at all: layouts that the kernels read in place do, others do not."""
+    import flash_pop_b200 as fp
+    from flash_pop_b200 import layer_ops
+    B, T, H, d = 2, 24, 3, 64
+    decays = tuple(orc.head_decays(H, (5, 12)))
+    pick = lambda: _layouts(torch.randn(B, T, H, d, device="cuda").to(dtype))[layout].detach().requires_grad_(True)
+    s = None if state is None else torch.randn(B, H, d, d, device="cuda").to(state)
+    x, dy = [pick() for _ in range(3)], pick().detach()
+    in_place = layout not in ("expanded", "inner")
+    with recorded() as taken:
+        o, _ = fp.fused_chunk_retention(*x, s, decays)
+        torch.autograd.grad(o, x, dy)
+        _, blocks = fp.flash_pop_retention(*x, s, decays, 8)
+        y = [t.detach().unsqueeze(1).requires_grad_(True) for t in x]
+        so = fp.pop_suffix_retention(*y, s, blocks.detach(), decays)
+        torch.autograd.grad(so, y, dy.unsqueeze(1))
+        fp.retention_step(*(t.detach()[:, 0] for t in x), decays, s)
+    assert taken == {"forward": [in_place] * 2, "backward": [in_place], "suffix_forward": [in_place], "suffix_backward": [in_place],
+                     "step": [in_place]}
+    with recorded() as taken:
+        torch.autograd.grad(layer_ops.rotary_qk(x[0], x[1], torch.randn(1, T, d // 2, 2, device="cuda")), x[:2], (dy, dy))
+        torch.autograd.grad(layer_ops.groupnorm_gate(x[0], x[1], 1e-6), x[:2], dy)
+        w = torch.randn(d, device="cuda")
+        torch.autograd.grad(layer_ops.layer_norm(x[0], w, w, 1e-6), x[:1], dy)
+    aligned = in_place and layout != "odd"
+    assert taken == {"rotary": [aligned] * 2, "gate_forward": [aligned], "gate_backward": [aligned], "norm_forward": [layout == "plain"],
+                     "norm_backward": [layout == "plain"]}
+
+
+def test_streams_and_threads():
+    """The extension releases the interpreter lock around the C ABI: threads on streams of their own, and a side stream of
+    the main thread, get what the main thread gets on its stream."""
+    import threading
+    import flash_pop_b200 as fp
+    decays = tuple(orc.head_decays(4, (5, 12)))
+    cases = []
+    for B, T, d, dtype in ((2, 300, 64, BF), (1, 2000, 128, BF), (2, 100, 32, F32)):
+        x = [(torch.randn(B, T, 4, d, device="cuda") * 0.1).to(dtype) for _ in range(4)]
+        cases.append((x, torch.randn(B, 4, d, d, device="cuda").to(dtype)))
+
+    def once(x, s):
+        leaves = [t.detach().requires_grad_(True) for t in x[:3]]
+        o, s_out = fp.fused_chunk_retention(*leaves, s, decays)
+        p, blocks = fp.flash_pop_retention(*leaves, s, decays, 16)
+        grads = torch.autograd.grad((o, p), leaves, (x[3], x[3]))
+        return [o.detach(), s_out.detach(), p.detach(), blocks.detach(), *grads, *fp.retention_step(*(t[:, 0] for t in x[:3]), decays, s)]
+
+    want = [once(*c) for c in cases]
+    torch.cuda.synchronize()
+    failures = []
+
+    def work(case, stream):
+        try:
+            with torch.cuda.stream(stream):
+                for _ in range(20):
+                    got = once(*cases[case])
+                    stream.synchronize()
+                    assert all(torch.equal(a, b) for a, b in zip(got, want[case]))
+        except BaseException as e:       # noqa: BLE001 - reported by the main thread
+            failures.append(e)
+
+    threads = [threading.Thread(target=work, args=(i % len(cases), torch.cuda.Stream())) for i in range(6)]
+    for t in threads:
+        t.start()
+    work(0, torch.cuda.Stream())
+    for t in threads:
+        t.join(120)
+    assert not failures, failures[0]

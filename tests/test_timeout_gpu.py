@@ -61,3 +61,33 @@ def test_wait_limit_runs_out_and_the_context_survives(d, dv, backward):
     o2, _, _ = step()
     _lib.device_status()
     check("O (release build)", o2, o_ref, BF)
+
+
+@pytest.mark.parametrize("rows", [3, 40])          # 40: the rows are normalised by a few CTAs, behind a barrier of its own
+def test_the_token_kernels_grid_barrier_gives_up_and_the_context_survives(rows):
+    """A wait of one cycle: the first CTAs to arrive at the grid barrier of ``fpb_decoder_token`` find it incomplete, report
+    it and leave, and so does everyone else; the launch returns and the next one is right."""
+    import ctypes
+    import flash_pop_b200 as fp
+    from flash_pop_b200 import _lib
+    torch.manual_seed(0)
+    cfg = fp.RetNetDecoderLayer.Config(num_heads=4, head_dim_v=64, dim_feedforward=256, dropout=0.0, device="cuda", dtype=BF)
+    net = fp.RetNetDecoder(cfg, 2).eval().requires_grad_(False)
+    x = torch.randn(rows, 256, device="cuda").to(BF)
+    stream = _lib.stream_ptr(torch.device("cuda"))
+    with torch.no_grad():
+        want, state = net.forward_recurrent(x)
+        with _lib.diagnostics_build() as diag:
+            detail = ctypes.c_int32(0)
+            try:
+                diag.fpb_debug_tuning(1, 200, 1, -1)
+                before = diag.fpb_launch_count()
+                net.forward_recurrent(x)
+                assert diag.fpb_launch_count() == before + 1           # the one launch, not the layers one by one
+                assert diag.fpb_device_status(stream, ctypes.byref(detail)) == 9 and detail.value == 0x7f0
+                assert diag.fpb_device_status(stream, ctypes.byref(detail)) == 0
+            finally:
+                diag.fpb_debug_tuning(0, 0, 1, -1)
+            got, state2 = net.forward_recurrent(x)
+            _lib.device_status()
+        assert torch.equal(got, want) and torch.equal(state2.state, state.state)
