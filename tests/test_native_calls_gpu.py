@@ -184,13 +184,14 @@ def test_the_extension_takes_the_ordinary_call(layout, dtype, state):
         fp.retention_step(*(t.detach()[:, 0] for t in x), decays, s)
     assert taken == {"forward": [in_place] * 2, "backward": [in_place], "suffix_forward": [in_place], "suffix_backward": [in_place],
                      "step": [in_place]}
+    if layout == "odd":                # (the layer passes refuse what 16-byte accesses cannot read)
+        return
     with recorded() as taken:
         torch.autograd.grad(layer_ops.rotary_qk(x[0], x[1], torch.randn(1, T, d // 2, 2, device="cuda")), x[:2], (dy, dy))
         torch.autograd.grad(layer_ops.groupnorm_gate(x[0], x[1], 1e-6), x[:2], dy)
         w = torch.randn(d, device="cuda")
         torch.autograd.grad(layer_ops.layer_norm(x[0], w, w, 1e-6), x[:1], dy)
-    aligned = in_place and layout != "odd"
-    assert taken == {"rotary": [aligned] * 2, "gate_forward": [aligned], "gate_backward": [aligned], "norm_forward": [layout == "plain"],
+    assert taken == {"rotary": [in_place] * 2, "gate_forward": [in_place], "gate_backward": [in_place], "norm_forward": [layout == "plain"],
                      "norm_backward": [layout == "plain"]}
 
 
