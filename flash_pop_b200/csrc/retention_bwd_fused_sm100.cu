@@ -145,13 +145,6 @@ __global__ void __launch_bounds__(BCfg<DK, DV>::NTHREADS, 1) bwd_fused_kernel(co
   // (Grouping of suffixes is compiled into the 64 x 64 kernel only - the shape suffixes come in; in the larger tiles its few
   // extra live registers spill the state, which costs the long-sequence workloads far more than grouping gains.)
   constexpr bool GROUPED = DK == 64 && DV == 64;
-  // (token, batch) coordinates in the tensor maps: grouped suffixes are batch entries of their own there, so that rows past
-  // a suffix's end read as zeros and are clipped on store
-  auto place = [&](int a) {
-    if (!GROUPED || p.sfx_G <= 1) return make_int2(a, b);
-    const int f = a / p.block_size;
-    return make_int2(a - f * p.block_size, f);
-  };
   auto stage_of = [&](int n) { return n % G::STAGES; };
   auto stage_ph = [&](int n) { return (uint32_t)((n / G::STAGES) & 1); };
   // tensor-memory addresses (lane offset in the upper half-word)
@@ -190,15 +183,24 @@ __global__ void __launch_bounds__(BCfg<DK, DV>::NTHREADS, 1) bwd_fused_kernel(co
   if (warp == 0) {                                   // ---------------- TMA producer
     if (lane == 0 && NC > 0) {
       Chunk ck = first;
+      // (token, batch) in the maps of what is read: grouped suffixes are batch entries of their own there, so rows past a
+      // suffix's end are zeros
+      int2 at = make_int2(ck.a, b);
+      if (GROUPED && p.sfx_G > 1) { at.y = ck.a / p.block_size; at.x -= at.y * p.block_size; }
+      auto next = [&]() {
+        const int a = ck.a;
+        prev_chunk(ck, p.block_size);
+        at.x -= a - ck.a;
+        if (GROUPED && at.x < 0) { at.x += p.block_size; --at.y; }     // (of grouped suffixes: into the one before)
+      };
       int issued = 0;
       for (int c = 0; c < NC; ++c) {
         const int s = stage_of(c);
         if (!mbar_wait(bar(B_EMPTY + s), stage_ph(c) ^ 1, abort_flag)) { FPB_GIVE_UP(0x100 | B_EMPTY); break; }
         FPB_TRACE(14, c);
-        if (c == p.tune.withhold_chunk) { prev_chunk(ck, p.block_size); continue; }   // diagnostics: this chunk never arrives
+        if (c == p.tune.withhold_chunk) { next(); continue; }   // diagnostics: this chunk never arrives
         const uint32_t st = sbase + G::OFF_STAGE + s * G::STAGE_BYTES;
         mbar_arrive_expect_tx(bar(B_FULL + s), G::STAGE_BYTES);
-        const int2 at = place(ck.a);
 #pragma unroll
         for (int cb = 0; cb < DV / 64; ++cb) {      // dO first: it has to be scaled before anything can use it
           tma_load_4d(st + G::OFF_DO + cb * 8192, &p.map_do, bar(B_FULL + s), vcol + cb * 64, at.x, h, at.y);
@@ -210,7 +212,7 @@ __global__ void __launch_bounds__(BCfg<DK, DV>::NTHREADS, 1) bwd_fused_kernel(co
           tma_load_4d(st + G::OFF_K + cb * 8192, &p.map_k, bar(B_FULL + s), cb * 64, at.x, h, at.y);
         }
         ++issued;
-        prev_chunk(ck, p.block_size);
+        next();
       }
       if (*abort_flag) {   // let the copies in flight land before the CTA's shared memory is released
         for (int i = max(0, issued - G::STAGES); i < issued && p.tune.withhold_chunk < 0; ++i) {
@@ -405,21 +407,19 @@ __global__ void __launch_bounds__(BCfg<DK, DV>::NTHREADS, 1) bwd_fused_kernel(co
       const float z_lo = exp2f((float)(ck.L - 1 - r_lo) * lg) * rs, z_hi = exp2f((float)(ck.L - 9 - r_lo) * lg) * rs;
       acc_to_staging(tm_accv, sm + G::OFF_OUTV, DV, z_lo, z_hi, false);
       acc_to_staging(tm_acck, sm + G::OFF_OUTK, DK, z_lo, z_hi, true);
-      // rows beyond L are past the end of the sequence, or of the suffix: TMA clips them
-      const bool whole_box = ck.L == C || ck.a + ck.L >= p.T || (GROUPED && p.sfx_G > 1);
+      const bool whole_box = ck.L == C || ck.a + ck.L >= p.T;
       if (whole_box) fence_async_smem();
       named_bar_sync(2, N_SCORE);
       if (whole_box) {
         if (t == 0) {
-          const int2 at = place(ck.a);
 #pragma unroll
-          for (int cb = 0; cb < DV / 64; ++cb) tma_store_4d(&p.map_dv, sbase + G::OFF_OUTV + cb * 8192, vcol + cb * 64, at.x, h, at.y);
+          for (int cb = 0; cb < DV / 64; ++cb) tma_store_4d(&p.map_dv, sbase + G::OFF_OUTV + cb * 8192, vcol + cb * 64, ck.a, h, b);
           if (p.dk_add) {
 #pragma unroll
-            for (int cb = 0; cb < DK / 64; ++cb) tma_reduce_add_4d(&p.map_dk, sbase + G::OFF_OUTK + cb * 8192, cb * 64, at.x, h, at.y);
+            for (int cb = 0; cb < DK / 64; ++cb) tma_reduce_add_4d(&p.map_dk, sbase + G::OFF_OUTK + cb * 8192, cb * 64, ck.a, h, b);
           } else {
 #pragma unroll
-            for (int cb = 0; cb < DK / 64; ++cb) tma_store_4d(&p.map_dk, sbase + G::OFF_OUTK + cb * 8192, cb * 64, at.x, h, at.y);
+            for (int cb = 0; cb < DK / 64; ++cb) tma_store_4d(&p.map_dk, sbase + G::OFF_OUTK + cb * 8192, cb * 64, ck.a, h, b);
           }
           tma_store_commit();
         }
@@ -812,8 +812,8 @@ int launch_bwd_fused(const UmmaBwdArgs& a, cudaStream_t stream, int* n_launched)
   if ((r = make_seq_map(&p.map_k, k, a.B, a.T, H, a.dk, C)) != FPB_OK) return r;
   if ((r = make_seq_map(&p.map_v, v, a.B, a.T, H, a.dv, C)) != FPB_OK) return r;
   if ((r = make_seq_map(&p.map_do, dO, a.B, a.T, H, a.dv, C)) != FPB_OK) return r;
-  if ((r = make_seq_map(&p.map_dk, dK, a.B, a.T, H, a.dk, C)) != FPB_OK) return r;
-  if ((r = make_seq_map(&p.map_dv, dV, a.B, a.T, H, a.dv, C)) != FPB_OK) return r;
+  if ((r = make_seq_map(&p.map_dk, dK, B, T, H, a.dk, C)) != FPB_OK) return r;
+  if ((r = make_seq_map(&p.map_dv, dV, B, T, H, a.dv, C)) != FPB_OK) return r;
   if (a.dk == 64 && a.dv == 64 && !a.state_f32 && a.d_block_states && a.n_blocks > 0) {
     // (B, N, H, dk, dv) contiguous as a 4-D tensor of 64-wide rows: dk rows per (block, head), N * H of those per batch row
     const SeqView bg{const_cast<void*>(a.d_block_states), (int64_t)a.n_blocks * H * a.dk * a.dv, (int64_t)a.dv, (int64_t)a.dk * a.dv};

@@ -224,14 +224,6 @@ scan_kernel(const __grid_constant__ ScanParams p) {
   const float rs = rsqrtf((float)p.dk);
   const int NC = chunk_count(t_end - t0, p.sched_bs);
   auto bar = [&](int slot) { return sbase + G::OFF_BAR + slot * 8; };
-  // (token, batch) coordinates in the tensor maps of the chunk that starts at token a of this walk.  Grouped suffixes stay
-  // batch entries of their own there: rows past a suffix's end read as zeros and are clipped on store.  (In a map over the
-  // joined sequence they were the next suffix's tokens, and an infinity in one reached the other through zero weights.)
-  auto place = [&](int a) {
-    if (p.sfx_G <= 1) return make_int2(a, b);
-    const int f = a / p.block_size;
-    return make_int2(a - f * p.block_size, f);
-  };
   constexpr int ARR_SCORE = N_SCORE, ARR_STATE = G::N_STATE;   // every thread of a role arrives (one elected lane per warp
                                                                 // after a warp sync was measured: no faster)
   auto warp_arrive = [&](uint32_t b_) { mbar_arrive(b_); };
@@ -279,16 +271,27 @@ scan_kernel(const __grid_constant__ ScanParams p) {
   if (warp == 0) {                                   // ---------------- TMA producer
     if (lane == 0 && NC > 0) {
       Chunk ck = first;
+      // Grouped suffixes are batch entries of their own in the maps of what is read, so rows past a suffix's end are zeros.
+      // (In a map over the joined sequence they were the next suffix's tokens, and an infinity in one reached the other
+      // through zero weights.)
+      constexpr bool GROUPED = !REV && !SO;
+      const bool grouped = GROUPED && p.sfx_G > 1;
+      int2 at = grouped ? make_int2(0, first.a / p.block_size) : make_int2(first.a, b);      // (token, batch) in the maps
+      auto next = [&]() {
+        const int a = ck.a;
+        advance<REV>(ck, t_end, p.sched_bs);
+        at.x += ck.a - a;
+        if (GROUPED && grouped && at.x >= p.block_size) { at.x = 0; ++at.y; }
+      };
       int issued = 0;
       for (int c = 0; c < NC; ++c) {
         const int s = stage_of(c);
         if (!mbar_wait(bar(B_EMPTY + s), stage_ph(c) ^ 1, abort_flag)) { FPB_GIVE_UP(0x100 | B_EMPTY); break; }
         FPB_TRACE(14, c);
-        if (c == p.tune.withhold_chunk) { advance<REV>(ck, t_end, p.sched_bs); continue; }   // diagnostics: this chunk never arrives
+        if (c == p.tune.withhold_chunk) { next(); continue; }   // diagnostics: this chunk never arrives
         const uint32_t st = sbase + G::OFF_STAGE + s * G::STAGE_BYTES;
         mbar_arrive_expect_tx(bar(B_FULL + s), SO ? G::K_BYTES + G::V_BYTES : G::STAGE_BYTES);
         const int xcol0 = MODE == MODE_FWD ? row0 : col0;
-        const int2 at = place(ck.a);
         if (!SO) {
 #pragma unroll
           for (int cb = 0; cb < G::W1 / 64; ++cb) tma_load_4d(st + cb * 8192, &p.map_x, bar(B_FULL + s), xcol0 + cb * 64, at.x, h, at.y);
@@ -298,7 +301,7 @@ scan_kernel(const __grid_constant__ ScanParams p) {
 #pragma unroll
         for (int cb = 0; cb < CC / 64; ++cb) tma_load_4d(st + G::X_BYTES + G::K_BYTES + cb * 8192, &p.map_v, bar(B_FULL + s), col0 + cb * 64, at.x, h, at.y);
         ++issued;
-        advance<REV>(ck, t_end, p.sched_bs);
+        next();
       }
       if (*abort_flag) {   // let the copies in flight land before the CTA's shared memory is released
         // (with a withheld chunk the stage numbering of the last copies is off by one: those were consumed anyway)
@@ -662,23 +665,21 @@ FPB_UNROLL_MMA
           *reinterpret_cast<uint32_t*>(stg + half * 8192 + (r_lo + 8) * 128 + ((g ^ ((r_lo + 8) & 7)) << 4) + cpair * 2) = hi;
         }
       }
-      // rows beyond L are past the end of the sequence, or of the suffix: TMA clips them
-      const bool whole_box = ck.L == C || ck.a + ck.L >= p.T || p.sfx_G > 1;
+      const bool whole_box = ck.L == C || ck.a + ck.L >= p.T;    // rows beyond L are past the sequence end: TMA clips them
       const int wrow0 = q4 * 16;                                // this warp's rows [wrow0, wrow0 + 16)
       const int ocol0 = MODE == MODE_FWD ? col0 : row0;
       if (whole_box) {
         if (!FPB_ABL(64)) fence_async_smem();
         __syncwarp();
-        if (lane == 0 && wrow0 < ck.L) {
-          const int2 at = place(ck.a);
+        if (lane == 0 && ck.a + wrow0 < p.T) {
           if (MODE == MODE_DQ && p.col_split == 1) {
 #pragma unroll
             for (int cb = 0; cb < G::NOUT / 64; ++cb)
-              tma_reduce_add_4d(&p.map_out, sbase + G::OFF_OUT + cb * 8192 + wrow0 * 128, ocol0 + cb * 64, at.x + wrow0, h, at.y);
+              tma_reduce_add_4d(&p.map_out, sbase + G::OFF_OUT + cb * 8192 + wrow0 * 128, ocol0 + cb * 64, ck.a + wrow0, h, b);
           } else {
 #pragma unroll
             for (int cb = 0; cb < G::NOUT / 64; ++cb)
-              tma_store_4d(&p.map_out, sbase + G::OFF_OUT + cb * 8192 + wrow0 * 128, ocol0 + cb * 64, at.x + wrow0, h, at.y);
+              tma_store_4d(&p.map_out, sbase + G::OFF_OUT + cb * 8192 + wrow0 * 128, ocol0 + cb * 64, ck.a + wrow0, h, b);
           }
           tma_store_commit();
         }
@@ -1285,7 +1286,7 @@ int launch_one(const PassArgs& a, Segments sg, bool state_only, cudaStream_t str
   if ((r = make_seq_map(&p.map_x, x, B, T, H, xw, C)) != FPB_OK) return r;
   if ((r = make_seq_map(&p.map_k, k, B, T, H, dk, C)) != FPB_OK) return r;
   if ((r = make_seq_map(&p.map_v, v, B, T, H, dv, C)) != FPB_OK) return r;
-  if ((r = make_seq_map(&p.map_out, out, B, T, H, ow, 16)) != FPB_OK) return r;   // one score warp's 16 rows
+  if ((r = make_seq_map(&p.map_out, out, Bk, Tk, H, ow, 16)) != FPB_OK) return r;   // one score warp's 16 rows
   p.out = (bf16*)out.data; p.out_sb = out.sb; p.out_st = out.st; p.out_sh = out.sh;
   const bool split = sg.n > 1 && a.sfx.M == 0;
   // a segmented walk starts from the scratch slots; its last piece writes the end value
