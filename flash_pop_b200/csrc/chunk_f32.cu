@@ -75,6 +75,7 @@ template <int DK, int DV> __device__ __forceinline__ void store_state(const floa
   }
 }
 
+// (padding of S, rows from dk and columns from dv on, stays the zero it was loaded as)
 // S <- decay S + sum over the chunk's n tokens of w_j A_j (x) B_j, w_j = pw[first + step * j]; a thread holds a
 // (DK/16) x (DV/16) block of S, rows side by side, columns in pieces of four
 template <int DK, int DV> __device__ __forceinline__ void update_state(float* S, const float* A, const float* B, const float* pw, int n,
@@ -102,13 +103,14 @@ template <int DK, int DV> __device__ __forceinline__ void update_state(float* S,
 #pragma unroll
       for (int c = 0; c < TC; ++c) acc[r][c] = fmaf(a[r], b[c], acc[r][c]);
   }
+  const bool all = dk == DK && dv == DV;
 #pragma unroll
   for (int r = 0; r < TR; ++r)
 #pragma unroll
     for (int c = 0; c < TC; ++c) {
       const int col = (c / CV) * (DV / NC) + c % CV;
       float& x = s0[r * (DV + 4) + col];
-      if (ty * TR + r < dk && tx * CV + col < dv) x = fmaf(decay, x, acc[r][c]);
+      if (all || (ty * TR + r < dk && tx * CV + col < dv)) x = fmaf(decay, x, acc[r][c]);
     }
 }
 
@@ -151,13 +153,12 @@ template <int R> __device__ __forceinline__ void add_to(float (&acc)[R][4], cons
 #pragma unroll
     for (int c = 0; c < 4; ++c) acc[r][c] += sum[r][c];
 }
-// acc += A[row] M  for the [K][N] matrix M (pitch N + 4), of which the first `real` (a multiple of 4) rows count
-template <int K, int N> __device__ __forceinline__ void times(float (&acc)[N / 32][4], const float* A, const float* M, const Own<N>& own, int real) {
-  for (int k0 = 0; k0 < real; k0 += 32) {
+// acc += A[row] M  for the [K][N] matrix M (pitch N + 4)
+template <int K, int N> __device__ __forceinline__ void times(float (&acc)[N / 32][4], const float* A, const float* M, const Own<N>& own) {
+  for (int k0 = 0; k0 < K; k0 += 32) {
     float sum[N / 32][4] = {};
-    const int k1 = min(k0 + 32, real);
 #pragma unroll 2
-    for (int k = k0; k < k1; k += 4) {
+    for (int k = k0; k < k0 + 32; k += 4) {
       float4 m[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) m[i] = *reinterpret_cast<const float4*>(M + (k + i) * (N + 4) + own.col);
@@ -175,13 +176,12 @@ template <int K, int N> __device__ __forceinline__ void times(float (&acc)[N / 3
     add_to<N / 32>(acc, sum);
   }
 }
-// acc += A[row] M^T for the [N][K] matrix M (pitch K + 4, `real` columns of it), columns N/4 apart
-template <int K, int N> __device__ __forceinline__ void times_t(float (&acc)[N / 32][4], const float* A, const float* M, const Own<N>& own, int real) {
-  for (int k0 = 0; k0 < real; k0 += 32) {
+// acc += A[row] M^T for the [N][K] matrix M (pitch K + 4), columns N/4 apart
+template <int K, int N> __device__ __forceinline__ void times_t(float (&acc)[N / 32][4], const float* A, const float* M, const Own<N>& own) {
+  for (int k0 = 0; k0 < K; k0 += 32) {
     float sum[N / 32][4] = {};
-    const int k1 = min(k0 + 32, real);
 #pragma unroll 2
-    for (int k = k0; k < k1; k += 4) {
+    for (int k = k0; k < k0 + 32; k += 4) {
       float4 m[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) m[i] = *reinterpret_cast<const float4*>(M + (own.col + i * (N / 4)) * (K + 4) + k);
@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(THREADS) chunk_fwd_kernel(const __grid_constan
     __syncthreads();
     scores<DK, false>(P, Q, K, pw);
     float acc[DV / 32][4] = {};
-    times<DK, DV>(acc, Q, S, own, p.dk);
+    times<DK, DV>(acc, Q, S, own);
     scale_rows<DV>(acc, own, pw, 1, 1, n);
     __syncthreads();
     times_scores<DV, false, false>(acc, P, V, own, n);
@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(THREADS) chunk_bwd_kernel(const __grid_constan
     if (!rev) {
       scores<DV, false>(P2, D, V, pw);
       float acc[DK / 32][4] = {};
-      times_t<DV, DK>(acc, D, S, own_k, p.dv);
+      times_t<DV, DK>(acc, D, S, own_k);
       scale_rows<DK>(acc, own_k, pw, 1, 1, n);
       __syncthreads();
       times_scores<DK, true, false>(acc, P2, K, own_k, n);
@@ -395,10 +395,10 @@ __global__ void __launch_bounds__(THREADS) chunk_bwd_kernel(const __grid_constan
       scores<DK, true>(P1, K, Q, pw);              // (K carries rs)
       scores<DV, true>(P2, V, D, pw);
       float av[DV / 32][4] = {};
-      times<DK, DV>(av, K, S, own_v, p.dk);
+      times<DK, DV>(av, K, S, own_v);
       scale_rows<DV>(av, own_v, pw, n - 1, -1, n);
       float ak[DK / 32][4] = {};
-      times_t<DV, DK>(ak, V, S, own_k, p.dv);
+      times_t<DV, DK>(ak, V, S, own_k);
       scale_rows<DK>(ak, own_k, pw, n - 1, -1, n);
       __syncthreads();
       times_scores<DV, false, true>(av, P1, D, own_v, n);
