@@ -788,7 +788,7 @@ int launch_bwd_fused(const UmmaBwdArgs& a, cudaStream_t stream, int* n_launched)
   if (a.sfx_grad.M > 0 && a.block_size == 0 && a.dk == 64 && a.dv == 64 && (int64_t)B * T <= (1 << 30)) {
     bool joined = true;
     for (const SeqView* s : {&q, &k, &v, &dO, &dK, &dV}) joined = joined && (B == 1 || s->sb == (int64_t)T * s->st);
-    if (joined) G = choose_suffix_group(B, H, 1);
+    if (joined) G = choose_suffix_group(B, T, H, 1);
     if (G > 1) {
       sg = Segments{(B + G - 1) / G, G * T};
       block_size = T; T *= B; B = 1;

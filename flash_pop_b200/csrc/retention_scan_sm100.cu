@@ -52,7 +52,7 @@
 // Suffix calls (thousands of sequences of a few chunks, each starting from its own state and dropping its end
 // state) may be regrouped by the launcher: where all suffixes of the call follow one another in memory they are ONE
 // sequence per head, cut into pieces of G suffixes (block size = suffix length, the state replaced at every suffix
-// start) - same results, and as many CTAs as fit the GPU at once, each with its even share.
+// start) - same results, with an even share for every CTA (choose_suffix_group).
 //
 // dv = 256 beside dk = 128.  A MODE_DQ walk may cut dv instead of dk (ScanParams::col_split): two CTAs per head on the
 // 128 x 128 instance, each with its half of the state columns; its output tile is then a partial sum, which the TMA
@@ -1176,7 +1176,7 @@ int launch_scan(const ScanParams& p, bool rev, bool state_only, dim3 grid, cudaS
 #endif
 FPB_KNOB g_tile_pref = 1;            // 1: 128x128 state tiles where they apply; 0: 64-wide tiles (two CTAs per SM)
 FPB_KNOB g_sfx_group = 1 << 20;      // most suffixes one CTA walks back to back (1: one CTA per suffix)
-FPB_KNOB g_sfx_slots = 0;            // CTAs they are shared out over (0: what fits the GPU at once)
+FPB_KNOB g_sfx_slots = 0;            // CTAs taken to run at once (0: what fits the GPU)
 FPB_KNOB g_pop_emit = 1;             // 1: POP forward walks over full chunks where block states can come from partial increments
 FPB_KNOB g_fused_bwd = 1;            // 1: dK, dV, dS_0 in one fused reverse walk where it applies; 0: two separate walks
 FPB_KNOB g_segments = 1;             // 1: under-filled launches are cut into T-segments when the caller gave scratch memory
@@ -1277,7 +1277,7 @@ int launch_one(const PassArgs& a, Segments sg, bool state_only, cudaStream_t str
   int Bk = B, Tk = T, block_size = a.block_size;
   auto joined = [&](const SeqView& s) { return B == 1 || s.sb == (int64_t)T * s.st; };
   if (a.sfx.M > 0 && !a.rev && a.block_size == 0 && (int64_t)B * T <= kMaxJoinedTokens && joined(x) && joined(k) && joined(v) && joined(out)) {
-    G = choose_suffix_group(B, (long long)H * t.tiles, t.ctas_per_sm);
+    G = choose_suffix_group(B, T, (long long)H * t.tiles, t.ctas_per_sm);
     if (G > 1) {
       sg = Segments{(B + G - 1) / G, G * T};
       Bk = 1; Tk = B * T; block_size = T;
@@ -1372,16 +1372,34 @@ void launch_zero_seq(const SeqView& v, int B, int T, int H, int d, cudaStream_t 
 }
 
 
-// The CTAs that fit the GPU at once, dealt out over the heads and tiles, share the suffixes evenly.  (Before, a CTA took a
-// divisor of M, at most 16, that left three waves: 1024 suffixes of 80 tokens per head, 8 heads, d = 64 were 8 a CTA in 3.46
-// waves, i.e. 32 suffixes a slot instead of 28 and four set-ups instead of one: forward 180 -> 156 us, dQ 166 -> 147.)
-// One each where that fits: no grouping.
-int choose_suffix_group(int suffixes, long long units, int ctas_per_sm) {
+// The CTAs that fit the GPU at once, dealt out over the heads and tiles (`units`), share the suffixes evenly - in one wave, or
+// in as many as it takes to leave few of them idle: a wave costs its suffixes' chunks and a set-up worth two, and the fewest
+// waves within 2 % of the cheapest number are taken (beyond 16 nothing is left to gain).  Measured, 1024 suffixes of 80 tokens
+// a head, d = 64, forward | backward in us, a divisor of M up to 16 in at least three waves / always one wave / this rule:
+//   heads    8: 187 | 412    173 | 385    177 | 386       56: 1115 | 2481   1132 | 2871   1093 | 2424
+//           20: 424 | 932    415 | 925    422 | 912       75: 1439 | 3228   1810 | 5244   1454 | 3261
+//   160 (512 suffixes): 1578 | 3472   2748 | 6108   1579 | 3487
+// One suffix each where that fits: no grouping.
+int choose_suffix_group(int suffixes, int tokens, long long units, int ctas_per_sm) {
   if (g_sfx_group <= 1) return 1;
+  constexpr int WAVES = 16, SET_UP = 2;
   const long long slots = g_sfx_slots > 0 ? g_sfx_slots : (long long)sm_count_cached() * ctas_per_sm;
-  long long n = slots / units;
-  if (n < 1) n = 1;
-  const long long G = (suffixes + n - 1) / n;
+  const long long chunks = (tokens + C - 1) / C;
+  long long group[WAVES], cost[WAVES], least = 0;
+  int n = 0;
+  for (int w = 1; w <= WAVES; ++w) {
+    long long pieces = w * slots / units;
+    if (pieces < 1) continue;
+    if (pieces > suffixes) pieces = suffixes;
+    const long long G = (suffixes + pieces - 1) / pieces, used = ((suffixes + G - 1) / G * units + slots - 1) / slots;
+    group[n] = G; cost[n] = used * (G * chunks + SET_UP);
+    if (n == 0 || cost[n] < least) least = cost[n];
+    ++n;
+    if (pieces == suffixes) break;
+  }
+  long long G = suffixes;                             // (more than 16 waves of whole heads)
+  for (int i = n - 1; i >= 0; --i)
+    if (cost[i] * 50 <= least * 51) G = group[i];
   return (int)(G < g_sfx_group ? G : g_sfx_group);
 }
 
@@ -1394,8 +1412,8 @@ extern "C" void fpb_debug_refuse_launch(int n) { g_refuse_launch = n; }
 extern "C" void fpb_debug_trace(void* device_buffer) { g_trace = (long long*)device_buffer; }
 // Choose between the 128x128 state tiles (1, default) and the 64-wide ones (0).
 extern "C" void fpb_debug_tile_pref(int wide) { g_tile_pref = wide; }
-// Upper limit of the suffixes one CTA walks back to back (1 = one CTA per suffix) and the number of CTAs they are shared out
-// over (0: what fits the GPU at once).
+// Upper limit of the suffixes one CTA walks back to back (1 = one CTA per suffix) and the number of CTAs taken to run at once
+// (0: what fits the GPU).
 extern "C" void fpb_debug_suffix_group(int g, int slots) { g_sfx_group = g < 1 ? 1 : g; g_sfx_slots = slots; }
 // 0 makes every POP forward walk cut its chunks at block ends.
 extern "C" void fpb_debug_pop_emit(int on) { g_pop_emit = on; }

@@ -47,8 +47,8 @@ bool col_split_enabled();
 bool halves_apart(long long heads);
 // zeros over the (B, T, H, d) bf16 elements of a strided view (d a multiple of 8, 16-byte aligned rows)
 void launch_zero_seq(const SeqView& v, int B, int T, int H, int d, cudaStream_t stream);
-// How many consecutive suffixes one CTA walks as one sequence; `units` = heads x tiles, each with all `suffixes`.
-int choose_suffix_group(int suffixes, long long units, int ctas_per_sm);
+// How many consecutive suffixes, of `tokens` each, one CTA walks as one sequence; `units` = heads x tiles, each with all of them.
+int choose_suffix_group(int suffixes, int tokens, long long units, int ctas_per_sm);
 // diagnostics: device buffer for per-chunk time stamps, or null
 long long* debug_trace_ptr();
 

@@ -52,3 +52,27 @@ def test_no_suffix_sees_the_next_one(P, dk, dv, bad):
         if m > 0:
             blocks[row, m - 1] = False
         assert torch.equal(got[5][blocks], clean[5][blocks])             # block states: where a later suffix starts
+
+
+@pytest.mark.parametrize("state_dtype", [BF, torch.float32])
+@pytest.mark.parametrize("B,M,N,P,H,dk,dv", [
+    (3, 50, 50, 80, 3, 64, 64), (7, 23, 22, 17, 5, 64, 64), (2, 75, 75, 64, 4, 64, 64), (5, 40, 41, 65, 2, 128, 128), (1, 200, 199, 80, 2, 64, 128),
+    (4, 40, 40, 16, 75, 64, 64), (3, 8, 8, 130, 160, 64, 64)])
+def test_the_shipped_sharing_equals_one_cta_per_suffix(B, M, N, P, H, dk, dv, state_dtype):
+    """Uneven pieces, pieces across batch rows, several waves of heads, both state types: bit for bit what one CTA per suffix
+    gives.  (Counts of suffixes and heads that the shipped rule groups; row by row, few suffixes a call, it does not.)"""
+    from flash_pop_b200 import _lib
+    decays = tuple(orc.head_decays(H, (5, 12)))
+    tensors, do = _case(B, M, N, P, H, dk, dv, state_dtype, seed=M)
+    grouped = _run(tensors, do, decays)
+    with _lib.diagnostics_build() as diag:
+        try:
+            diag.fpb_debug_suffix_group(1, 0)
+            single = _run(tensors, do, decays)
+        finally:
+            diag.fpb_debug_suffix_group(1 << 20, 0)
+    for a, b in zip(grouped, single):
+        assert torch.equal(a, b)
+    rows = orc.pop_suffix_retention(*(t[:1, :, :, :2].double().cpu() for t in tensors[:3]), tensors[3][:1, :2].double().cpu(),
+                                    tensors[4][:1, :, :2].double().cpu(), decays[:2])
+    assert orc.rel_rms(grouped[0][:1, :, :, :2].float().cpu(), rows) < 5e-3

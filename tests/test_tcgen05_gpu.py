@@ -222,8 +222,9 @@ def test_host_memory_pipeline_pop():
 
 @pytest.mark.parametrize("M,N,P,d", [(8, 8, 80, 64), (12, 12, 40, 64), (9, 8, 80, 64), (6, 6, 100, 128)])
 def test_grouped_suffix_walks_equal_one_cta_per_suffix(M, N, P, d):
-    """Consecutive suffixes of a row walked by one CTA as one sequence (state replaced at every suffix start) give
-    bit for bit what one CTA per suffix gives, forward and backward; odd counts and strided tensors fall back."""
+    """Consecutive suffixes of a call, across batch rows too, walked by one CTA as one sequence (state replaced at every
+    suffix start) give bit for bit what one CTA per suffix gives, forward and backward: one piece for all of them, and as
+    many as two CTAs share out."""
     import flash_pop_b200 as fp
     from flash_pop_b200 import _lib
     B, H = 2, 3
@@ -235,8 +236,8 @@ def test_grouped_suffix_walks_equal_one_cta_per_suffix(M, N, P, d):
     results = []
     with _lib.diagnostics_build() as diag:      # the schedule hooks exist in the diagnostics build only
         try:
-            for limit, floor in ((1, 1), (16, 1)):
-                diag.fpb_debug_suffix_group(limit, floor)
+            for limit, slots in ((1, 0), (1 << 20, H), (1 << 20, 2 * H)):
+                diag.fpb_debug_suffix_group(limit, slots)
                 leaves = [t.detach().clone().requires_grad_(True) for t in (sq, sk, sv, s0, blocks)]
                 o = fp.pop_suffix_retention(leaves[0], leaves[1], leaves[2], leaves[3], leaves[4], decays)
                 assert _lib.last_path() == _lib.PATH_TCGEN05
@@ -244,9 +245,9 @@ def test_grouped_suffix_walks_equal_one_cta_per_suffix(M, N, P, d):
                 results.append([o.detach()] + [t.grad for t in leaves])
             _lib.device_status()
         finally:
-            diag.fpb_debug_suffix_group(16, 3 * 296)
-    for a, b in zip(*results):
-        assert torch.equal(a, b)
+            diag.fpb_debug_suffix_group(1 << 20, 0)
+    for a, b, c in zip(*results):
+        assert torch.equal(a, b) and torch.equal(a, c)
     qd, kd, vd = (t.double().cpu() for t in (sq, sk, sv))
     o_ref = orc.pop_suffix_retention(qd, kd, vd, s0.double().cpu(), blocks.double().cpu(), decays)
     assert orc.rel_rms(results[1][0].float().cpu(), o_ref) < 5e-3
