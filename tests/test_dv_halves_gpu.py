@@ -37,3 +37,29 @@ def test_halves_apart_equal_halves_together(B, H, T, state):
             for i, (a, c) in enumerate(zip(whole, grads(slice(b, b + 1), heads))):
                 want = a[b:b + 1][:, :, heads] if i < 3 else a[b:b + 1][:, heads]
                 assert torch.equal(want, c)
+
+
+@pytest.mark.parametrize("B,H,apart", [(1, 74, False), (1, 75, True), (4, 37, True), (1, 149, False), (1, 222, False), (1, 223, True)])
+def test_which_calls_keep_the_halves_apart(B, H, apart):
+    """Apart where two launches of one half take no more waves than one of both: four launches of walks in the backward, the
+    last of which the diagnostics build can refuse; together there are two, over outputs zeroed first."""
+    import flash_pop_b200 as fp
+    from flash_pop_b200 import _lib
+    assert torch.cuda.get_device_properties(0).multi_processor_count == 148
+    decays = tuple(orc.head_decays(H, (5, 12)))
+    r = lambda d: (torch.randn(B, 70, H, d, device="cuda") * 0.1).bfloat16()
+    q, k, v, dO = r(128).requires_grad_(True), r(128).requires_grad_(True), r(256).requires_grad_(True), r(256)
+    with _lib.diagnostics_build() as diag:
+        try:
+            o, _ = fp.fused_chunk_retention(q, k, v, None, decays)
+            want = torch.autograd.grad(o, [q, k, v], dO, retain_graph=True)
+            diag.fpb_debug_refuse_launch(3)
+            if apart:
+                with pytest.raises(RuntimeError, match="launch"):
+                    torch.autograd.grad(o, [q, k, v], dO, retain_graph=True)
+            else:
+                got = torch.autograd.grad(o, [q, k, v], dO, retain_graph=True)
+                assert all(torch.equal(a, b) for a, b in zip(got, want))
+        finally:
+            diag.fpb_debug_refuse_launch(-1)
+    _lib.device_status()
