@@ -75,10 +75,10 @@ template <int DK, int DV> __device__ __forceinline__ void store_state(const floa
   }
 }
 
-// (padding of S, rows from dk and columns from dv on, stays the zero it was loaded as)
 // S <- decay S + sum over the chunk's n tokens of w_j A_j (x) B_j, w_j = pw[first + step * j]; a thread holds a
-// (DK/16) x (DV/16) block of S, rows side by side, columns in pieces of four
-template <int DK, int DV> __device__ __forceinline__ void update_state(float* S, const float* A, const float* B, const float* pw, int n,
+// (DK/16) x (DV/16) block of S, rows side by side, columns in pieces of four.  Padding of S - rows from dk, columns from dv
+// on, none where EXACT - stays the zero it was loaded as.
+template <int DK, int DV, bool EXACT> __device__ __forceinline__ void update_state(float* S, const float* A, const float* B, const float* pw, int n,
                                                                        int first, int step, float decay, int dk, int dv) {
   constexpr int TR = DK / 16, TC = DV / 16, CV = TC < 4 ? TC : 4, NC = TC / CV;
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
@@ -103,14 +103,13 @@ template <int DK, int DV> __device__ __forceinline__ void update_state(float* S,
 #pragma unroll
       for (int c = 0; c < TC; ++c) acc[r][c] = fmaf(a[r], b[c], acc[r][c]);
   }
-  const bool all = dk == DK && dv == DV;
 #pragma unroll
   for (int r = 0; r < TR; ++r)
 #pragma unroll
     for (int c = 0; c < TC; ++c) {
       const int col = (c / CV) * (DV / NC) + c % CV;
       float& x = s0[r * (DV + 4) + col];
-      if (all || (ty * TR + r < dk && tx * CV + col < dv)) x = fmaf(decay, x, acc[r][c]);
+      if (EXACT || (ty * TR + r < dk && tx * CV + col < dv)) x = fmaf(decay, x, acc[r][c]);
     }
 }
 
@@ -200,9 +199,9 @@ template <int N, bool STRIDED, bool UP> __device__ __forceinline__ void times_sc
                                                                                     const Own<N>& own, int n) {
   constexpr int R = N / 32;
   float sum[R][4] = {};
-  const int lo = UP ? own.row & ~3 : 0, hi = UP ? (n + 3) & ~3 : (own.row + R + 3) & ~3;
+  const int lo = UP ? own.row & ~3 : 0, hi = UP ? n & ~3 : (own.row + R + 3) & ~3;
   for (int k = lo; k < hi; k += 4) {
-    const bool whole = UP ? k >= own.row + R - 1 && k + 3 < n : k + 3 <= own.row;
+    const bool whole = UP ? k >= own.row + R - 1 : k + 3 <= own.row;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       float4 m;
@@ -212,11 +211,23 @@ template <int N, bool STRIDED, bool UP> __device__ __forceinline__ void times_sc
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const int row = own.row + r;
-        if (whole || (UP ? k + i >= row && k + i < n : k + i <= row)) {
+        if (whole || (UP ? k + i >= row : k + i <= row)) {
           const float e = P[row * PP + k + i];
           sum[r][0] = fmaf(e, m.x, sum[r][0]); sum[r][1] = fmaf(e, m.y, sum[r][1]);
           sum[r][2] = fmaf(e, m.z, sum[r][2]); sum[r][3] = fmaf(e, m.w, sum[r][3]);
         }
+      }
+    }
+  }
+  if (UP) {                                        // the last, broken group of four of a ragged chunk
+    for (int k = max(hi, lo); k < n; ++k) {
+      const float* mr = M + k * (N + 4) + own.col;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        if (k < own.row + r) continue;
+        const float e = P[(own.row + r) * PP + k];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) sum[r][c] = fmaf(e, mr[STRIDED ? c * (N / 4) : c], sum[r][c]);
       }
     }
   }
@@ -258,7 +269,7 @@ __device__ __forceinline__ float* slot_of(float* base, const ChunkParams& p, int
 
 // Local end values of the segments, from zero: grid (n_seg - 1, H, roles * B).  Role 0: the state over (k, v), every
 // segment but the last; role 1: its gradient over (q, dO), every segment but the first.
-template <int DK, int DV>
+template <int DK, int DV, bool EXACT>
 __global__ void __launch_bounds__(THREADS) chunk_segments_kernel(const __grid_constant__ ChunkParams p) {
   using M = Smem<DK, DV>;
   extern __shared__ __align__(16) float sm[];
@@ -274,7 +285,7 @@ __global__ void __launch_bounds__(THREADS) chunk_segments_kernel(const __grid_co
     load_tile<DK>(A, rev ? p.q : p.k, b, h, a, n, p.dk, rev ? 1.0f : rs);
     load_tile<DV>(B, rev ? p.dO : p.v, b, h, a, n, p.dv, 1.0f);
     __syncthreads();
-    update_state<DK, DV>(S, A, B, pw, n, rev ? 1 : n - 1, rev ? 1 : -1, pw[n], p.dk, p.dv);
+    update_state<DK, DV, EXACT>(S, A, B, pw, n, rev ? 1 : n - 1, rev ? 1 : -1, pw[n], p.dk, p.dv);
     __syncthreads();
   }
   grid_wait();                                     // (the first of the chain: nothing to wait for)
@@ -323,7 +334,7 @@ __device__ __forceinline__ const float* start_of(const ChunkParams& p, float* sc
   return s.data ? (const float*)s.data + b * s.sb + h * s.sh : nullptr;
 }
 
-template <int DK, int DV>
+template <int DK, int DV, bool EXACT>
 __global__ void __launch_bounds__(THREADS) chunk_fwd_kernel(const __grid_constant__ ChunkParams p) {
   using M = Smem<DK, DV>;
   extern __shared__ __align__(16) float sm[];
@@ -351,14 +362,14 @@ __global__ void __launch_bounds__(THREADS) chunk_fwd_kernel(const __grid_constan
     __syncthreads();
     times_scores<DV, false, false>(acc, P, V, own, n);
     store_rows<DV, false>(acc, own, p.o, b, h, a, n, p.dv, 1.0f);
-    if (a + L32 < t1 || ends) update_state<DK, DV>(S, K, V, pw, n, n - 1, -1, pw[n], p.dk, p.dv);   // (S was last read before the barrier)
+    if (a + L32 < t1 || ends) update_state<DK, DV, EXACT>(S, K, V, pw, n, n - 1, -1, pw[n], p.dk, p.dv);   // (S was last read before the barrier)
     __syncthreads();
   }
   if (ends) store_state<DK, DV>(S, (float*)p.s_out.data + b * p.s_out.sb + h * p.s_out.sh, p.dk, p.dv);
 }
 
 // z-blocks below n_fwd: dQ (forward walk over the state); the others: dK, dV, dS_0 (reverse walk over its gradient)
-template <int DK, int DV>
+template <int DK, int DV, bool EXACT>
 __global__ void __launch_bounds__(THREADS) chunk_bwd_kernel(const __grid_constant__ ChunkParams p) {
   using M = Smem<DK, DV>;
   extern __shared__ __align__(16) float sm[];
@@ -390,7 +401,7 @@ __global__ void __launch_bounds__(THREADS) chunk_bwd_kernel(const __grid_constan
       __syncthreads();
       times_scores<DK, true, false>(acc, P2, K, own_k, n);
       store_rows<DK, true>(acc, own_k, p.dQ, b, h, a, n, p.dk, 1.0f);
-      if (c + 1 < chunks) update_state<DK, DV>(S, K, V, pw, n, n - 1, -1, pw[n], p.dk, p.dv);
+      if (c + 1 < chunks) update_state<DK, DV, EXACT>(S, K, V, pw, n, n - 1, -1, pw[n], p.dk, p.dv);
     } else {
       scores<DK, true>(P1, K, Q, pw);              // (K carries rs)
       scores<DV, true>(P2, V, D, pw);
@@ -405,7 +416,7 @@ __global__ void __launch_bounds__(THREADS) chunk_bwd_kernel(const __grid_constan
       store_rows<DV, false>(av, own_v, p.dV, b, h, a, n, p.dv, 1.0f);
       times_scores<DK, true, true>(ak, P2, Q, own_k, n);
       store_rows<DK, true>(ak, own_k, p.dK, b, h, a, n, p.dk, rs);
-      if (c + 1 < chunks || (seg == 0 && p.g_out.data)) update_state<DK, DV>(S, Q, D, pw, n, 1, 1, pw[n], p.dk, p.dv);
+      if (c + 1 < chunks || (seg == 0 && p.g_out.data)) update_state<DK, DV, EXACT>(S, Q, D, pw, n, 1, 1, pw[n], p.dk, p.dv);
     }
     __syncthreads();
   }
@@ -417,7 +428,7 @@ cudaError_t launch(void (*kernel)(ChunkParams), dim3 grid, size_t smem, bool cha
 }
 
 enum Pass { SEGMENTS, FORWARD, BACKWARD };
-template <int DK, int DV>
+template <int DK, int DV, bool EXACT>
 cudaError_t launch_pass_t(Pass pass, dim3 grid, bool chained, const ChunkParams& p, cudaStream_t stream) {
   using M = Smem<DK, DV>;
   static_assert(M::BWD <= 227 * 1024, "shared memory of a CTA");
@@ -426,20 +437,22 @@ cudaError_t launch_pass_t(Pass pass, dim3 grid, bool chained, const ChunkParams&
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(chunk_segments_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, M::TILES2)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(chunk_fwd_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, M::FWD)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(chunk_bwd_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, M::BWD)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(chunk_segments_kernel<DK, DV, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, M::TILES2)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(chunk_fwd_kernel<DK, DV, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, M::FWD)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(chunk_bwd_kernel<DK, DV, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, M::BWD)) != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
   }
-  if (pass == SEGMENTS) return launch(chunk_segments_kernel<DK, DV>, grid, M::TILES2, chained, p, stream);
-  if (pass == FORWARD) return launch(chunk_fwd_kernel<DK, DV>, grid, M::FWD, chained, p, stream);
-  return launch(chunk_bwd_kernel<DK, DV>, grid, M::BWD, chained, p, stream);
+  if (pass == SEGMENTS) return launch(chunk_segments_kernel<DK, DV, EXACT>, grid, M::TILES2, chained, p, stream);
+  if (pass == FORWARD) return launch(chunk_fwd_kernel<DK, DV, EXACT>, grid, M::FWD, chained, p, stream);
+  return launch(chunk_bwd_kernel<DK, DV, EXACT>, grid, M::BWD, chained, p, stream);
 }
 cudaError_t launch_pass(Pass pass, dim3 grid, bool chained, const ChunkParams& p, cudaStream_t stream) {
   auto tile = [](int d) { return d <= 32 ? 32 : d <= 64 ? 64 : 128; };
   const int key = tile(p.dk) * 1000 + tile(p.dv);
+  const bool exact = tile(p.dk) == p.dk && tile(p.dv) == p.dv;
   switch (key) {
-#define FPB_CHUNK_CASE(DK_, DV_) case DK_ * 1000 + DV_: return launch_pass_t<DK_, DV_>(pass, grid, chained, p, stream)
+#define FPB_CHUNK_CASE(DK_, DV_) case DK_ * 1000 + DV_: \
+    return exact ? launch_pass_t<DK_, DV_, true>(pass, grid, chained, p, stream) : launch_pass_t<DK_, DV_, false>(pass, grid, chained, p, stream)
     FPB_CHUNK_CASE(32, 32); FPB_CHUNK_CASE(32, 64); FPB_CHUNK_CASE(32, 128);
     FPB_CHUNK_CASE(64, 32); FPB_CHUNK_CASE(64, 64); FPB_CHUNK_CASE(64, 128);
     FPB_CHUNK_CASE(128, 32); FPB_CHUNK_CASE(128, 64); FPB_CHUNK_CASE(128, 128);
