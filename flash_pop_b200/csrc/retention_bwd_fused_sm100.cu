@@ -183,36 +183,32 @@ __global__ void __launch_bounds__(BCfg<DK, DV>::NTHREADS, 1) bwd_fused_kernel(co
   if (warp == 0) {                                   // ---------------- TMA producer
     if (lane == 0 && NC > 0) {
       Chunk ck = first;
-      // (token, batch) in the maps of what is read: grouped suffixes are batch entries of their own there, so rows past a
+      // batch entry in the maps of what is read and its first token: grouped suffixes are entries of their own, so rows past a
       // suffix's end are zeros
-      int2 at = make_int2(ck.a, b);
-      if (GROUPED && p.sfx_G > 1) { at.y = ck.a / p.block_size; at.x -= at.y * p.block_size; }
-      auto next = [&]() {
-        const int a = ck.a;
-        prev_chunk(ck, p.block_size);
-        at.x -= a - ck.a;
-        if (GROUPED && at.x < 0) { at.x += p.block_size; --at.y; }     // (of grouped suffixes: into the one before)
-      };
+      int entry = b, entry_t0 = 0;
+      if (GROUPED && p.sfx_G > 1) { entry = ck.a / p.block_size; entry_t0 = entry * p.block_size; }
       int issued = 0;
       for (int c = 0; c < NC; ++c) {
         const int s = stage_of(c);
         if (!mbar_wait(bar(B_EMPTY + s), stage_ph(c) ^ 1, abort_flag)) { FPB_GIVE_UP(0x100 | B_EMPTY); break; }
         FPB_TRACE(14, c);
-        if (c == p.tune.withhold_chunk) { next(); continue; }   // diagnostics: this chunk never arrives
+        if (c == p.tune.withhold_chunk) { prev_chunk(ck, p.block_size); continue; }   // diagnostics: this chunk never arrives
         const uint32_t st = sbase + G::OFF_STAGE + s * G::STAGE_BYTES;
         mbar_arrive_expect_tx(bar(B_FULL + s), G::STAGE_BYTES);
+        if (GROUPED && ck.a < entry_t0) { --entry; entry_t0 -= p.block_size; }
+        const int at = GROUPED ? ck.a - entry_t0 : ck.a;
 #pragma unroll
         for (int cb = 0; cb < DV / 64; ++cb) {      // dO first: it has to be scaled before anything can use it
-          tma_load_4d(st + G::OFF_DO + cb * 8192, &p.map_do, bar(B_FULL + s), vcol + cb * 64, at.x, h, at.y);
-          tma_load_4d(st + G::OFF_V + cb * 8192, &p.map_v, bar(B_FULL + s), vcol + cb * 64, at.x, h, at.y);
+          tma_load_4d(st + G::OFF_DO + cb * 8192, &p.map_do, bar(B_FULL + s), vcol + cb * 64, at, h, entry);
+          tma_load_4d(st + G::OFF_V + cb * 8192, &p.map_v, bar(B_FULL + s), vcol + cb * 64, at, h, entry);
         }
 #pragma unroll
         for (int cb = 0; cb < DK / 64; ++cb) {
-          tma_load_4d(st + G::OFF_Q + cb * 8192, &p.map_q, bar(B_FULL + s), cb * 64, at.x, h, at.y);
-          tma_load_4d(st + G::OFF_K + cb * 8192, &p.map_k, bar(B_FULL + s), cb * 64, at.x, h, at.y);
+          tma_load_4d(st + G::OFF_Q + cb * 8192, &p.map_q, bar(B_FULL + s), cb * 64, at, h, entry);
+          tma_load_4d(st + G::OFF_K + cb * 8192, &p.map_k, bar(B_FULL + s), cb * 64, at, h, entry);
         }
         ++issued;
-        next();
+        prev_chunk(ck, p.block_size);
       }
       if (*abort_flag) {   // let the copies in flight land before the CTA's shared memory is released
         for (int i = max(0, issued - G::STAGES); i < issued && p.tune.withhold_chunk < 0; ++i) {

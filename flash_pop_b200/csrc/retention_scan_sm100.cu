@@ -275,33 +275,29 @@ scan_kernel(const __grid_constant__ ScanParams p) {
       // (In a map over the joined sequence they were the next suffix's tokens, and an infinity in one reached the other
       // through zero weights.)
       constexpr bool GROUPED = !REV && !SO;
-      const bool grouped = GROUPED && p.sfx_G > 1;
-      int2 at = grouped ? make_int2(0, first.a / p.block_size) : make_int2(first.a, b);      // (token, batch) in the maps
-      auto next = [&]() {
-        const int a = ck.a;
-        advance<REV>(ck, t_end, p.sched_bs);
-        at.x += ck.a - a;
-        if (GROUPED && grouped && at.x >= p.block_size) { at.x = 0; ++at.y; }
-      };
+      int entry = b, entry_t0 = 0, entry_end = 0x7fffffff;       // batch entry in the maps, its first token and its end
+      if (GROUPED && p.sfx_G > 1) { entry = seg * p.sfx_G; entry_t0 = t0; entry_end = t0 + p.block_size; }
       int issued = 0;
       for (int c = 0; c < NC; ++c) {
         const int s = stage_of(c);
         if (!mbar_wait(bar(B_EMPTY + s), stage_ph(c) ^ 1, abort_flag)) { FPB_GIVE_UP(0x100 | B_EMPTY); break; }
         FPB_TRACE(14, c);
-        if (c == p.tune.withhold_chunk) { next(); continue; }   // diagnostics: this chunk never arrives
+        if (c == p.tune.withhold_chunk) { advance<REV>(ck, t_end, p.sched_bs); continue; }   // diagnostics: this chunk never arrives
         const uint32_t st = sbase + G::OFF_STAGE + s * G::STAGE_BYTES;
         mbar_arrive_expect_tx(bar(B_FULL + s), SO ? G::K_BYTES + G::V_BYTES : G::STAGE_BYTES);
         const int xcol0 = MODE == MODE_FWD ? row0 : col0;
+        if (GROUPED && ck.a >= entry_end) { ++entry; entry_t0 = entry_end; entry_end += p.block_size; }
+        const int at = GROUPED ? ck.a - entry_t0 : ck.a;
         if (!SO) {
 #pragma unroll
-          for (int cb = 0; cb < G::W1 / 64; ++cb) tma_load_4d(st + cb * 8192, &p.map_x, bar(B_FULL + s), xcol0 + cb * 64, at.x, h, at.y);
+          for (int cb = 0; cb < G::W1 / 64; ++cb) tma_load_4d(st + cb * 8192, &p.map_x, bar(B_FULL + s), xcol0 + cb * 64, at, h, entry);
         }
 #pragma unroll
-        for (int cb = 0; cb < R / 64; ++cb) tma_load_4d(st + G::X_BYTES + cb * 8192, &p.map_k, bar(B_FULL + s), row0 + cb * 64, at.x, h, at.y);
+        for (int cb = 0; cb < R / 64; ++cb) tma_load_4d(st + G::X_BYTES + cb * 8192, &p.map_k, bar(B_FULL + s), row0 + cb * 64, at, h, entry);
 #pragma unroll
-        for (int cb = 0; cb < CC / 64; ++cb) tma_load_4d(st + G::X_BYTES + G::K_BYTES + cb * 8192, &p.map_v, bar(B_FULL + s), col0 + cb * 64, at.x, h, at.y);
+        for (int cb = 0; cb < CC / 64; ++cb) tma_load_4d(st + G::X_BYTES + G::K_BYTES + cb * 8192, &p.map_v, bar(B_FULL + s), col0 + cb * 64, at, h, entry);
         ++issued;
-        next();
+        advance<REV>(ck, t_end, p.sched_bs);
       }
       if (*abort_flag) {   // let the copies in flight land before the CTA's shared memory is released
         // (with a withheld chunk the stage numbering of the last copies is off by one: those were consumed anyway)
