@@ -462,7 +462,11 @@ cudaError_t launch_pass(Pass pass, dim3 grid, bool chained, const ChunkParams& p
 }
 
 // Segments of whole chunks: as many as the CTAs that fit the GPU at once (one an SM at 128 wide, two below), each at
-// least one chunk; no more than the scratch holds.
+// least one chunk; no more than the scratch holds; none where they do not pay.  In tenths of a chunk a sequence costs 10 a
+// chunk whole, in segments 16 a chunk of one (state pass and walk) and 30 where they fill the GPU.  Measured, forward | backward
+// in us, whole against split: 64 heads, d = 64, T = 33 14.7 | 20.1 against 23.6 | 31.0 (the token walk 18.3 | 51.3), T = 160
+// 36.4 | 55.6 against 45.1 | 62.3, T = 300 70.0 | 107 against 69.8 | 104, T = 1024 223 | 405 against 184 | 303; 8 heads, T = 96
+// 21.8 | 33.7 against 14.0 | 18.5; 64 heads, d = 128, T = 300 140 | 233 against 114 | 258, T = 1024 570 | 873 against 431 | 879.
 void choose(ChunkParams& p, int64_t scratch_bytes, int directions) {
   const int chunks = (p.T + L32 - 1) / L32;
   const int64_t units = (int64_t)p.B * p.H, slots = 148 * ((p.dk > 64 && p.dv > 64) ? 1 : 2);
@@ -474,8 +478,10 @@ void choose(ChunkParams& p, int64_t scratch_bytes, int directions) {
   n = n < chunks ? n : chunks;
   p.n_seg = 1; p.seg_len = chunks * L32;
   if (n < 2) return;
-  p.seg_len = (int)((chunks + n - 1) / n) * L32;
-  p.n_seg = (p.T + p.seg_len - 1) / p.seg_len;
+  const int per = (int)((chunks + n - 1) / n), count = (chunks + per - 1) / per;
+  if (16 * per + 30 * units * count / slots >= 10 * chunks) return;
+  p.seg_len = per * L32;
+  p.n_seg = count;
 }
 
 bool seq_ok(const SeqView& s, int B, int T, int H) {
