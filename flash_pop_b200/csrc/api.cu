@@ -735,7 +735,8 @@ int64_t fpb_workspace_bytes(const fpb_dims* dims) {
   // (the small state tiles run two CTAs per SM: ask for what that residency can use)
   const int ctas_per_sm = (dims->dk <= 64 || dims->dv <= 64) ? 2 : 1;
   const Segments sg = choose_segments((long long)dims->B * dims->H, ctas_per_sm, dims->T, 64, (long long)dims->B * dims->H,
-                                      (long long)dims->dk * dims->dv, 0, dims->B);
+                                      (long long)dims->dk * dims->dv, 0, dims->B,
+                                      dims->dv == 128 ? kPairedChunkDq128 : kPairedChunk);      // (the dQ walk splits furthest)
   return sg.n > 1 ? (int64_t)dims->B * dims->H * sg.n * dims->dk * dims->dv * 4 : 0;
 }
 int fpb_last_path(void) { return tl_last_path; }

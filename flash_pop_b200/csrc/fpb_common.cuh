@@ -122,8 +122,10 @@ struct Segments {
 };
 // `units` CTAs the launch would have unsplit, `ctas_per_sm` of them resident per SM; `align` = token count every
 // segment start must be a multiple of; state_floats = dk * dv; scratch holds B*H*n*state_floats floats.
+// `paired`: what a chunk of a piece costs where an SM gets two CTAs (segment_scan.cu).
+constexpr int kPairedChunk = 400, kPairedChunkDq128 = 270;
 Segments choose_segments(long long units, int ctas_per_sm, int T, int align, long long batch_heads, long long state_floats,
-                         long long scratch_bytes, int B);
+                         long long scratch_bytes, int B, int paired = kPairedChunk);
 int sm_count();              // of the current device
 // Start values of the segments from the local end values of all but the piece reached last: in place over `seg`
 // (B, H, n, dk, dv) fp32.

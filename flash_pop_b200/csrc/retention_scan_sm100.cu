@@ -1324,7 +1324,7 @@ int launch_pass(const PassArgs& a, cudaStream_t stream, int* n_launched) {
     const Tiling t = tiling_of(a.mode, a.dk, a.dv, col_split_ok(a.mode, a.block_size, a.sfx));
     const int align = a.block_size > 0 ? C / gcd_int(C, a.block_size) * a.block_size : C;   // segment starts: chunk and block multiples
     sg = choose_segments((long long)t.tiles * a.H * a.B, t.ctas_per_sm, a.T, align, (long long)a.B * a.H, (long long)a.dk * a.dv,
-                         a.scratch_bytes, a.B);
+                         a.scratch_bytes, a.B, a.mode == MODE_DQ && t.CC == 128 ? kPairedChunkDq128 : kPairedChunk);
   }
   int r;
   if (sg.n > 1) {
