@@ -262,8 +262,9 @@ using namespace fpb;
 #define FPB_TRY(expr) do { const int _s = (expr); if (_s != FPB_OK) return _s; } while (0)
 
 namespace {
-// What decides whether fpb_retention_fwd_static takes a shape: the scratch of pieces of at least 512 tokens.  Within the
-// built-in scratch a call is split as far as that allows.  (fp32 calls are taken whatever their size.)
+// What decides whether fpb_retention_fwd_static takes a shape: the scratch of pieces of at least 512 tokens, which is what the
+// entry point has refused by since it came - finer pieces (choose_segments) need more, but nobody has to have them.  Within
+// the built-in scratch a call is split as far as that allows.  (fp32 calls are taken whatever their size.)
 int64_t static_split_bytes(const fpb_dims& d) {
   if (d.dtype != FPB_BF16 || d.B <= 0 || d.H <= 0) return 0;
   const int64_t units = (int64_t)d.B * d.H, slots = (int64_t)sm_count() * ((d.dk <= 64 || d.dv <= 64) ? 2 : 1);
@@ -719,7 +720,7 @@ const char* fpb_strerror(int status) {
     case FPB_ERR_DEVICE_TIMEOUT: return "a bounded wait inside a kernel gave up";
     case FPB_ERR_TENSOR_MAP: return "could not encode a TMA tensor map for a tensor";
     case FPB_ERR_TOO_LARGE: return "size beyond a fixed limit of this entry point (batch over 65535, or more scratch than the built-in array holds)";
-    case FPB_ERR_BAD_WORKSPACE: return "workspace pointer not 16-byte aligned or negative size";
+    case FPB_ERR_BAD_WORKSPACE: return "workspace pointer not 16-byte aligned, or its size negative or less than the call needs";
     default: return "unknown status";
   }
 }

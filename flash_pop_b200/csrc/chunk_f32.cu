@@ -469,7 +469,7 @@ cudaError_t launch_pass(Pass pass, dim3 grid, bool chained, const ChunkParams& p
 // 21.8 | 33.7 against 14.0 | 18.5; 64 heads, d = 128, T = 300 140 | 233 against 114 | 258, T = 1024 570 | 873 against 431 | 879.
 void choose(ChunkParams& p, int64_t scratch_bytes, int directions) {
   const int chunks = (p.T + L32 - 1) / L32;
-  const int64_t units = (int64_t)p.B * p.H, slots = 148 * ((p.dk > 64 && p.dv > 64) ? 1 : 2);
+  const int64_t units = (int64_t)p.B * p.H, slots = (int64_t)sm_count() * ((p.dk > 64 && p.dv > 64) ? 1 : 2);
   int64_t n = units > 0 ? slots / units : 1;
   if (scratch_bytes >= 0) {
     const int64_t fit = scratch_bytes / (units * p.dk * p.dv * 4 * directions);

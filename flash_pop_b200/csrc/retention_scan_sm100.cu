@@ -1127,16 +1127,6 @@ int launch_scan_t(const ScanParams& p, dim3 grid, cudaStream_t stream) {
   const bool chained = !SO && p.n_seg > 1 && p.sfx_M == 0;      // behind the scan over its segments
   return launch_kernel(scan_kernel<MODE, REV, R, CC, SO, SF32, DEEP>, grid, G::NTHREADS, G::SMEM, chained, p, stream) == cudaSuccess ? FPB_OK : FPB_ERR_LAUNCH;
 }
-int sm_count_cached() {
-  static std::atomic<int> cache[64];
-  int dev = 0, n = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if ((n = cache[dev].load(std::memory_order_acquire)) == 0) {
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    cache[dev].store(n, std::memory_order_release);
-  }
-  return n;
-}
 
 #ifdef FPB_DIAGNOSTICS
 int g_deep = 1;                  // 1: small tiles take the deep-pipeline variant when the grid has at most one CTA per SM
@@ -1156,7 +1146,7 @@ int launch_scan(const ScanParams& p, bool rev, bool state_only, dim3 grid, cudaS
   }
   if (state_only) return FPB_ERR_BAD_SHAPE;
   if constexpr (R == 64 && CC == 64) {   // at most one CTA per SM: the deep-pipeline variant (forward walks, bf16 states)
-    if (!f32 && !rev && g_deep && (long long)grid.x * grid.y * grid.z <= sm_count_cached())
+    if (!f32 && !rev && g_deep && (long long)grid.x * grid.y * grid.z <= sm_count())
       return launch_scan_t<MODE, 0, R, CC, false, false, true>(p, grid, stream);
   }
   if (f32) return rev ? launch_scan_t<MODE, 1, R, CC, false, true>(p, grid, stream) : launch_scan_t<MODE, 0, R, CC, false, true>(p, grid, stream);
@@ -1355,10 +1345,12 @@ const WalkTuning& walk_tuning() { return g_tuning; }
 bool segments_enabled() { return g_segments != 0; }
 // The two halves of dv as launches of their own, where that takes no more waves of one CTA an SM than one launch of both:
 // the first then stores its partial results and only the second adds, so the zero fill of the output goes (81 us of 537 MB
-// each for dQ and dK at B = 4, H = 32, T = 16384; reading K and Q twice gives part of it back: the whole training call 3582 ->
-// 3540 us).  Same results: adding to a zero is exact.
+// each for dQ and dK at B = 4, H = 32, T = 16384; reading K and Q twice gives part of it back).  Backward, together -> apart in
+// us, medians of 11 alternating runs in one process: 128 heads T = 16384 2497 -> 2374, T = 4096 617 -> 586, T = 1024 228 -> 217;
+// 75 heads T = 8192 1099 -> 1047, 87 heads T = 16384 2185 -> 2043, 100 heads T = 8192 1141 -> 1054, 148 heads 1442 -> 1322.
+// Same results: adding to a zero is exact.
 bool halves_apart(long long heads) {
-  const long long sms = sm_count_cached(), both = (2 * heads + sms - 1) / sms;
+  const long long sms = sm_count(), both = (2 * heads + sms - 1) / sms;
   return heads * 2 > sms && 2 * ((heads + sms - 1) / sms) <= both;
 }
 bool col_split_enabled() { return g_col_split != 0 && g_tile_pref != 0; }
@@ -1379,7 +1371,7 @@ void launch_zero_seq(const SeqView& v, int B, int T, int H, int d, cudaStream_t 
 int choose_suffix_group(int suffixes, int tokens, long long units, int ctas_per_sm) {
   if (g_sfx_group <= 1) return 1;
   constexpr int WAVES = 16, SET_UP = 2;
-  const long long slots = g_sfx_slots > 0 ? g_sfx_slots : (long long)sm_count_cached() * ctas_per_sm;
+  const long long slots = g_sfx_slots > 0 ? g_sfx_slots : (long long)sm_count() * ctas_per_sm;
   const long long chunks = (tokens + C - 1) / C;
   long long group[WAVES], cost[WAVES], least = 0;
   int n = 0;

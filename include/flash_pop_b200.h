@@ -42,7 +42,7 @@ typedef enum fpb_status {
   FPB_ERR_DEVICE_TIMEOUT = 9,  /* a bounded in-kernel wait gave up (reported by fpb_device_status) */
   FPB_ERR_TENSOR_MAP = 10,     /* cuTensorMapEncodeTiled refused the tensor */
   FPB_ERR_TOO_LARGE = 11,      /* size beyond a fixed limit of this entry point */
-  FPB_ERR_BAD_WORKSPACE = 12   /* workspace pointer misaligned or size negative */
+  FPB_ERR_BAD_WORKSPACE = 12   /* workspace pointer misaligned, size negative or less than the call needs */
 } fpb_status;
 
 typedef enum fpb_dtype { FPB_BF16 = 0, FPB_F32 = 1 } fpb_dtype;
@@ -122,8 +122,9 @@ int fpb_copy_rows_async(void* dst, int64_t dst_pitch, const void* src, int64_t s
  * FPB_STATIC_SCRATCH_BYTES of device memory per GPU that loads the library, held until the process exits.
  *   - Inputs and outputs are the caller's as in fpb_retention_fwd; dims->workspace must be NULL.
  *   - The call itself allocates nothing and frees nothing (no cudaMalloc / cudaFree, no allocating library routine).
- *   - A shape whose split would use more scratch than the array holds (fpb_workspace_bytes(dims) >
- *     FPB_STATIC_SCRATCH_BYTES) is refused with FPB_ERR_TOO_LARGE; shapes that fill the GPU unsplit use no scratch.
+ *   - A bf16 shape whose split into pieces of 512 tokens and more would use more scratch than the array holds is refused
+ *     with FPB_ERR_TOO_LARGE; any other call is split as far as the array goes.  Shapes that fill the GPU unsplit
+ *     (fpb_workspace_bytes(dims) == 0) use no scratch.
  *   - The first call on each device looks up the array's device address (cudaGetSymbolAddress) and keeps it; make that
  *     first call outside any stream capture.
  *   - All calls on a device share the one array.  It keeps whatever the last call left; nothing in it has to start at
@@ -229,8 +230,8 @@ int64_t fpb_decoder_token_workspace(const fpb_token_dims* dims);
  * One token of every row through `layers` consecutive decoder layers (RetNetDecoder.forward_recurrent,
  * flash_pop/retnet.py:535-546; RetNetDecoderLayer.forward_recurrent and MultiScaleRetention.forward_recurrent below it):
  *   x <- x + out_proj(GroupNorm(retention step(rotate(q), rotate(k), v)) . act(gate)),   x <- x + linear2(act(linear1(norm(x))))
- * x, y: (B, H dv) bf16 rows, row pitches in elements.  At most 64 rows, H dv <= 1024 and a multiple of 32, ffn a multiple
- * of 32, H dk of 8, dv of 4, dk even; FPB_ERR_BAD_SHAPE outside.  One cooperative launch per 16 layers, no allocation, no
+ * x, y: (B, H dv) bf16 rows, row pitches in elements.  At most 64 rows, H dv <= 1024 (as fpb_layernorm_fwd takes bf16
+ * rows) and a multiple of 32, ffn a multiple of 32, H dk of 8, dv of 4, dk even; FPB_ERR_BAD_SHAPE outside.  One cooperative launch per 16 layers, no allocation, no
  * synchronisation with the host.
  */
 int fpb_decoder_token(const fpb_token_dims* dims, const fpb_decoder_layer* layers, const void* x, int64_t x_stride,
