@@ -87,16 +87,17 @@ int sm_count() {
 
 constexpr int kLongPiece = 512;          // tokens
 
-// What a walk costs, in hundredths of a microsecond (fitted to one B200, 1 to 32 heads in all, d = 64 and 128, T = 300 to 32768):
-// whole, 600 and 155 a chunk of its sequence; in pieces - state pass, scan and walk, three set-ups - 1400, 260 a chunk of a
-// piece (`paired` where an SM gets two CTAs: kPairedChunk, less in the 64 x 128 tiles of the dQ walk) and 27 a piece, which the
-// scan takes one after the other.  The two launches more are worth 600 of the host's time.  Both sides measured (forward, us): 8 heads, T = 1000, d = 128 whole 30.8, 8 pieces 22.7; 4
-// heads, T = 3000 in 5 pieces 41.1, in 24 26.3; but 16 heads, T = 600 whole 20.7, 4 pieces 24.7, 8 heads, T = 300 whole 13.7,
-// 2 pieces 22.7, and 32 heads, T = 777, d = 64 whole 22.8, 7 pieces 18.6, which a training call of 100 us of host work pays
-// with 10 us.  (Pieces of at least 512 tokens, the rule before the launches were chained, left the first two at 30.8 and 41.1.)
-// Forward | backward by pieces: 1 head, d = 64, T = 8192 in 16 26.8 | 53.9, in 32 21.4 | 43.8, in 128 31.6 | 65.3, T = 32768 in
-// 64 35.8 | 72.1, in 74 35.3 | 72.1, in 256 60.8 | 101; 2 heads, d = 128, T = 32768 in 64 48.3 | 106, in 74 55.0 | 119; 4 heads,
-// d = 64, T = 8192 in 32 22.0 | 44.8, in 64 26.6 | 49.9; 16 heads in 8 44.5 | 89.3, in 16 38.2 | 83.3.
+// What a walk costs, in hundredths of a microsecond (fitted to one B200, 1 to 32 heads in all, d = 64 and 128, T = 300 to
+// 32768): whole, 600 and 155 a chunk of its sequence; in pieces - state pass, scan and walk, three set-ups - 1400, 260 a chunk
+// of a piece (`paired` where an SM gets two CTAs: kPairedChunk, less in the 64 x 128 tiles of the dQ walk) and 27 a piece, which
+// the scan takes one after the other.  The two launches more are worth 600 of the host's time.  Both sides measured (forward,
+// us): 8 heads, T = 1000, d = 128 whole 30.8, 8 pieces 22.7; 4 heads, T = 3000 in 5 pieces 41.1, in 24 26.3; but 16 heads,
+// T = 600 whole 20.7, 4 pieces 24.7, 8 heads, T = 300 whole 13.7, 2 pieces 22.7, and 32 heads, T = 777, d = 64 whole 22.8, 7
+// pieces 18.6, which a training call of 100 us of host work pays with 10 us.  (Pieces of at least 512 tokens, the rule before
+// the launches were chained, left the first two at 30.8 and 41.1.)  Forward | backward by pieces: 1 head, d = 64, T = 8192 in 16
+// 26.8 | 53.9, in 32 21.4 | 43.8, in 128 31.6 | 65.3, T = 32768 in 64 35.8 | 72.1, in 74 35.3 | 72.1, in 256 60.8 | 101; 2 heads,
+// d = 128, T = 32768 in 64 48.3 | 106, in 74 55.0 | 119; 4 heads, d = 64, T = 8192 in 32 22.0 | 44.8, in 64 26.6 | 49.9; 16 heads
+// in 8 44.5 | 89.3, in 16 38.2 | 83.3.
 static long long cost_whole(int T) { return 600 + 155 * ((T + 63) / 64); }
 static long long cost_pieces(int seg_len, long long count, long long a_chunk) { return 1400 + a_chunk * ((seg_len + 63) / 64) + 27 * count; }
 constexpr int kLaunchesHost = 600;

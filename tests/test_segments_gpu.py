@@ -148,3 +148,34 @@ def test_workspace_is_optional_and_checked():
     assert call(buf.data_ptr(), two) == (0, 3)
     assert call(buf.data_ptr(), two - 16) == (0, 1)          # not even two pieces fit: walked whole
     _lib.device_status()
+
+
+@pytest.mark.parametrize("B,T,H,d,dtype,least,most", [
+    (1, 8192, 1, 64, BF, 16, 64), (1, 32768, 1, 64, BF, 48, 128), (1, 8192, 4, 128, BF, 24, 37), (1, 1000, 8, 128, BF, 8, 8), (1, 5003, 16, 128, BF, 9, 9),
+    (1, 300, 8, 128, BF, 0, 0), (4, 777, 8, 64, BF, 0, 0), (8, 33, 8, 64, torch.float32, 0, 0), (8, 160, 8, 64, torch.float32, 0, 0),
+    (2, 256, 4, 64, torch.float32, 8, 8), (8, 1024, 8, 64, torch.float32, 4, 4)])
+def test_how_far_calls_are_cut(B, T, H, d, dtype, least, most):
+    """The number of pieces by the scratch a call asks for: neither a piece a chunk, whose scan costs more than the walks,
+    nor cuts that do not pay; and what comes out either way is the same."""
+    import ctypes
+    from flash_pop_b200 import _lib
+    decays = orc.head_decays(H, (5, 12) if H > 1 else None)
+    q, k, v, s, g = make_inputs(T, B, T, H, d, d, dtype)
+    q, k, v, s = (t.cuda() for t in (q, k, v, s))
+    need = _lib.lib().fpb_workspace_bytes(ctypes.byref(_lib.dims(q, d, decays)))
+    pieces = need // (B * H * d * d * 4 * (2 if dtype == torch.float32 else 1))
+    assert least <= pieces <= most, pieces
+
+    def run(nbytes):
+        o, s_out = torch.empty_like(v), torch.empty_like(s)
+        dm, scratch = _lib.dims(q, d, decays), torch.empty(max(nbytes, 16), dtype=torch.uint8, device="cuda")
+        if nbytes:
+            dm.workspace, dm.workspace_bytes = scratch.data_ptr(), nbytes
+        _lib.check(_lib.lib().fpb_retention_fwd(dm, _lib.seq(q), _lib.seq(k), _lib.seq(v), _lib.state(s), _lib.seq(o), _lib.state(s_out),
+                                                _lib.stream_ptr(q.device)))
+        return o, s_out
+
+    # (fp32: sums of some 10^3 products in another order; bf16: the state's copies of 2^-9 from another fp32 rounding)
+    limit = 2e-6 if dtype == torch.float32 else 5e-3
+    for a, b in zip(run(need), run(0)):
+        assert orc.rel_rms(a.float().cpu(), b.double().cpu()) < limit
